@@ -258,6 +258,18 @@ static int create(fbse_ctx *c, const fbse_grid_desc *g, const double *pot, const
     axis_k2(ns[a], dk, ng_1, k);
     if ((rc = upload(c, dst[a], k.data(), k.size()))) return rc;
     if ((rc = upload(c, dstf[a], k.data(), k.size()))) return rc;
+    AxisPlan &p = c->ax[a];
+    if (p.P > 0) {  // the same table by the positions of a two-factor transform
+      std::vector<double> ko(k.size());
+      std::vector<int> ord(k.size());
+      for (int pos = 0; pos < p.n; pos++) {
+        ord[pos] = pos / p.P + p.Q * (pos % p.P);
+        ko[pos] = k[ord[pos]];
+      }
+      if ((rc = upload(c, &p.ord, ord.data(), ord.size()))) return rc;
+      if ((rc = upload(c, &p.k2o, ko.data(), ko.size()))) return rc;
+      if ((rc = upload(c, &p.k2of, ko.data(), ko.size()))) return rc;
+    }
   }
   if ((rc = upload(c, &c->pot64, pot, c->ngrid))) return rc;
   if ((rc = upload(c, &c->pot32, pot, c->ngrid))) return rc;

@@ -57,6 +57,15 @@ struct AxisPlan {
   int radix[kMaxStages] = {0};
   double2 *tw64 = nullptr;  // device, n roots e^{-2 pi i t / n}
   float2 *tw32 = nullptr;   // device, same roots rounded to FP32
+  // two-factor kernels (fft_two.cuh): n = P Q, 0 when the length has no such
+  // factors; twiddles e^{-2 pi i t k1 / n} at t + P k1, the k index of each
+  // position of a transformed line, and the kinetic table in that order
+  int P = 0, Q = 0;
+  double2 *two64 = nullptr;
+  float2 *two32 = nullptr;
+  int *ord = nullptr;
+  double *k2o = nullptr;
+  float *k2of = nullptr;
 };
 
 // ---------------------------------------------------------------------------

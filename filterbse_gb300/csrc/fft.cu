@@ -4,6 +4,10 @@
 // fftw_plan_dft_3d(nz, ny, nx) forward transform, the ksqr multiply and the
 // unnormalised backward transform (plans made in filter_mpi/aux.c:259-270).
 //
+// Axes of 64, 128 and 256 points take the register-resident kernels
+// (fft_fast.cuh), axes with two register radices the two-factor kernels
+// (fft_two.cuh); every other length, and fbse_tuning.fft_kernels = 1, takes the
+// kernels of this file:
 // Each axis is a self-sorting mixed-radix Stockham FFT on lines held in shared
 // memory.  The grid sizes the reference's auto-grid produces are arbitrary
 // (e.g. 57 x 52 x 45 = 3*19 x 4*13 x 9*5), so an axis is factored into
@@ -60,6 +64,25 @@ static std::vector<int> factorize(int n)
   return r;
 }
 
+// n = P Q for the two-factor kernels: both radices at most 16 and as close as
+// possible, else the largest P with a Q of the second set; false: neither
+static bool two_factors(int n, int *P, int *Q)
+{
+  for (int set = 0; set < 2; set++)
+    for (int p = 16; p >= 1; p--) {
+      const int q = n / p;
+      if (n % p || q < p) continue;
+      const bool second = q == 17 || q == 18 || q == 19 || q == 20 || q == 21 || q == 23 || q == 24 || q == 25 ||
+                          q == 29 || q == 31;
+      if (set == 0 ? q <= 16 : second) {
+        *P = p;
+        *Q = q;
+        return true;
+      }
+    }
+  return false;
+}
+
 int plan_axis(fbse_ctx *c, AxisPlan &p, int n)
 {
   if (n < 1) return set_err(c, FBSE_ERR_ARG, "grid axis must have at least one point");
@@ -81,15 +104,28 @@ int plan_axis(fbse_ctx *c, AxisPlan &p, int n)
   FBSE_CUDA(c, cudaMalloc(&p.tw32, n * sizeof(float2)));
   FBSE_CUDA(c, cudaMemcpy(p.tw64, h64.data(), n * sizeof(double2), cudaMemcpyHostToDevice));
   FBSE_CUDA(c, cudaMemcpy(p.tw32, h32.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
+  if (two_factors(n, &p.P, &p.Q)) {
+    std::vector<double2> t64(n);
+    std::vector<float2> t32(n);
+    for (int k1 = 0; k1 < p.Q; k1++)
+      for (int t = 0; t < p.P; t++) {
+        t64[t + p.P * k1] = h64[t * k1 % n];
+        t32[t + p.P * k1] = h32[t * k1 % n];
+      }
+    FBSE_CUDA(c, cudaMalloc(&p.two64, n * sizeof(double2)));
+    FBSE_CUDA(c, cudaMalloc(&p.two32, n * sizeof(float2)));
+    FBSE_CUDA(c, cudaMemcpy(p.two64, t64.data(), n * sizeof(double2), cudaMemcpyHostToDevice));
+    FBSE_CUDA(c, cudaMemcpy(p.two32, t32.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
+  }
   return FBSE_OK;
 }
 
 void free_axis(AxisPlan &p)
 {
-  if (p.tw64) cudaFree(p.tw64);
-  if (p.tw32) cudaFree(p.tw32);
-  p.tw64 = nullptr;
-  p.tw32 = nullptr;
+  void *bufs[] = {p.tw64, p.tw32, p.two64, p.two32, p.ord, p.k2o, p.k2of};
+  for (void *b : bufs)
+    if (b) cudaFree(b);
+  p = AxisPlan();
 }
 
 static Stages stages_of(const AxisPlan &p)
@@ -387,7 +423,7 @@ __global__ void __launch_bounds__(256, 4) k_fft_cols(C<T> *__restrict__ data, St
       // convolution: multiply by the k-space array (hartree, bse_cplx/hartree.c:19-27)
       for (int t = threadIdx.x; t < n * L; t += blockDim.x) {
         const int cc = t % L, i = t / L;
-        const double2 q = ka.kq[(long)i * ka.nxy + (long)jy * ka.nx + x0 + cc];
+        const double2 q = ka.kq[(long)i * ka.nxy + kin_xy(ka, x0 + cc, jy)];
         A[t] = cmul<T>(A[t], mk<T>((T)q.x, (T)q.y));
       }
     } else {
@@ -457,9 +493,17 @@ static int launch_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv,
   return FBSE_OK;
 }
 
+// the z pass's multiplier: the kinetic tables, or the k-space array kq, for x and
+// y positions in k order or (xo, yo) in a two-factor transform's order
+static KinArgs kin_args(fbse_ctx *c, const double2 *kq, bool xo, bool yo)
+{
+  const AxisPlan &x = c->ax[0], &y = c->ax[1];
+  return {xo ? x.k2o : c->k2x,   yo ? y.k2o : c->k2y,   c->k2z, xo ? x.k2of : c->k2xf, yo ? y.k2of : c->k2yf, c->k2zf,
+          c->kemax_scaled, kq, c->nx, c->nx * c->ny, xo ? x.ord : nullptr, yo ? y.ord : nullptr};
+}
+
 template <typename T>
-static int launch_cols(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, bool kmul,
-                       const double2 *kq = nullptr)
+static int launch_cols(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, bool kmul, const KinArgs &ka)
 {
   const AxisPlan &p = c->ax[axis];
   const int n = p.n;
@@ -483,7 +527,6 @@ static int launch_cols(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, b
   const size_t smem = (size_t)(n + (st.big ? 2L : 1L) * TX * n) * sizeof(C<T>);
   if (smem > (size_t)max_smem()) return set_err(c, FBSE_ERR_UNSUPPORTED, "FFT axis too long for shared memory");
   const long grid = nouter * nxt;
-  KinArgs ka{c->k2x, c->k2y, c->k2z, c->k2xf, c->k2yf, c->k2zf, c->kemax_scaled, kq, c->nx, c->nx * c->ny};
   if (kmul) {
     FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_cols<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_fft_cols<T, true><<<grid, 256, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1, s2,
@@ -596,7 +639,7 @@ static int launch_plane_fast(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, 
 }
 
 template <typename T, int N>
-static int launch_cols_fast_n(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, bool kmul, const double2 *kq)
+static int launch_cols_fast_n(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, bool kmul, const KinArgs &ka)
 {
   using Cfg = fast::ColsCfg<T, N>;
   const int nxt = (int)((c->nx + 31) / 32);
@@ -609,7 +652,6 @@ static int launch_cols_fast_n(fbse_ctx *c, C<T> *data, long nblk, int axis, bool
   const size_t smem = Cfg::smem();
   const long grid = nouter * nxt;
   const C<T> *rt = roots<T>(c->ax[axis]);
-  KinArgs ka{c->k2x, c->k2y, c->k2z, c->k2xf, c->k2yf, c->k2zf, c->kemax_scaled, kq, c->nx, c->nx * c->ny};
   if (kmul) {
     FBSE_CUDA(c, cudaFuncSetAttribute(fast::k_cols_fast<T, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
@@ -625,21 +667,28 @@ static int launch_cols_fast_n(fbse_ctx *c, C<T> *data, long nblk, int axis, bool
   return FBSE_OK;
 }
 
-template <typename T>
-static int launch_cols_any(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, bool kmul,
-                           const double2 *kq = nullptr)
+// two-factor kernels (fft_two.cuh): any other length that has the two factors
+static bool two_axis_ok(fbse_ctx *c, int axis)
 {
+  return c->tune.fft_kernels == 0 && c->ax[axis].P > 0 && !fast_axis_ok(c, c->ax[axis].n);
+}
+
+// y or z lines; z (kmul): forward, multiply, inverse
+template <typename T>
+static int launch_cols_any(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, bool kmul, const KinArgs &ka)
+{
+  if (two_axis_ok(c, axis)) return kmul ? two_z<T>(c, data, nblk, ka) : two_y<T>(c, data, nblk, inv);
   switch (fast_axis_ok(c, c->ax[axis].n) ? c->ax[axis].n : 0) {
-    case 64: return launch_cols_fast_n<T, 64>(c, data, nblk, axis, inv, kmul, kq);
-    case 128: return launch_cols_fast_n<T, 128>(c, data, nblk, axis, inv, kmul, kq);
-    case 256: return launch_cols_fast_n<T, 256>(c, data, nblk, axis, inv, kmul, kq);
-    default: return launch_cols<T>(c, data, nblk, axis, inv, kmul, kq);
+    case 64: return launch_cols_fast_n<T, 64>(c, data, nblk, axis, inv, kmul, ka);
+    case 128: return launch_cols_fast_n<T, 128>(c, data, nblk, axis, inv, kmul, ka);
+    case 256: return launch_cols_fast_n<T, 256>(c, data, nblk, axis, inv, kmul, ka);
+    default: return launch_cols<T>(c, data, nblk, axis, inv, kmul, ka);
   }
 }
 
 int zpass_kinetic(fbse_ctx *c, float2 *data, long nblk)
 {
-  return launch_cols_any<float>(c, data, nblk, 2, false, true);
+  return launch_cols_any<float>(c, data, nblk, 2, false, true, kin_args(c, nullptr, false, false));
 }
 
 template <typename T, int N>
@@ -668,6 +717,7 @@ template <typename T>
 static int launch_x_any(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, int epi, const C<T> *phi,
                         const T *pot, T ca, T cb)
 {
+  if (two_axis_ok(c, 0)) return two_x<T>(c, in, out, nblk, inv, phi, pot, ca, cb);
   switch (fast_axis_ok(c, c->nx) ? c->nx : 0) {
     case 64: return launch_x_fast_n<T, 64>(c, in, out, nblk, inv, epi, phi, pot, ca, cb);
     case 128: return launch_x_fast_n<T, 128>(c, in, out, nblk, inv, epi, phi, pot, ca, cb);
@@ -685,9 +735,17 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
 {
   int rc;
   const Stages sx = stages_of(c->ax[0]), sy = stages_of(c->ax[1]);
-  const bool plane = !sx.big && !sy.big && plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;
   const T *pot = with_v ? pot_of<T>(c) : nullptr;
   const bool fplane = fast_plane_ok<T>(c);
+  // a plane of two lengths that both have two factors (64, 128 and 256 do) when it fits
+  const bool tplane = !fplane && c->tune.fft_kernels == 0 && c->ax[0].P > 0 && c->ax[1].P > 0 &&
+                      two_plane_smem<T>(c) <= (size_t)max_smem();
+  const bool lines = two_axis_ok(c, 0) || two_axis_ok(c, 1);
+  const bool plane = !lines && !sx.big && !sy.big && plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;
+  // which of x and y the z pass meets in a two-factor transform's order
+  const bool xo = tplane || (!fplane && !plane && two_axis_ok(c, 0));
+  const bool yo = tplane || (!fplane && !plane && two_axis_ok(c, 1));
+  const KinArgs ka = kin_args(c, kq, xo, yo);
   for (long b0 = 0; b0 < nblk; b0 += cb) {
     const long nb = (nblk - b0 < cb) ? nblk - b0 : cb;
     const C<T> *ci = in + b0 * c->ngrid;
@@ -695,17 +753,21 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
     C<T> *wk = work;  // reused by every chunk: a chunk's intermediate passes can stay in L2
     if (fplane) {
       if ((rc = launch_plane_fast<T>(c, ci, wk, nb, 0, nullptr, nullptr, T(1), T(0)))) return rc;
-      if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, kq))) return rc;
+      if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, ka))) return rc;
       if ((rc = launch_plane_fast<T>(c, wk, co, nb, 1, ci, pot, (T)a, (T)b))) return rc;
+    } else if (tplane) {
+      if ((rc = two_plane<T>(c, ci, wk, nb, false, nullptr, nullptr, T(1), T(0)))) return rc;
+      if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, ka))) return rc;
+      if ((rc = two_plane<T>(c, wk, co, nb, true, ci, pot, (T)a, (T)b))) return rc;
     } else if (plane) {
       if ((rc = launch_plane<T>(c, ci, wk, nb, 0, nullptr, nullptr, T(1), T(0)))) return rc;
-      if ((rc = launch_cols<T>(c, wk, nb, 2, false, true, kq))) return rc;
+      if ((rc = launch_cols<T>(c, wk, nb, 2, false, true, ka))) return rc;
       if ((rc = launch_plane<T>(c, wk, co, nb, 1, ci, pot, (T)a, (T)b))) return rc;
     } else {
       if ((rc = launch_x_any<T>(c, ci, wk, nb, false, 0, nullptr, nullptr, T(1), T(0)))) return rc;
-      if ((rc = launch_cols_any<T>(c, wk, nb, 1, false, false))) return rc;
-      if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, kq))) return rc;
-      if ((rc = launch_cols_any<T>(c, wk, nb, 1, true, false))) return rc;
+      if ((rc = launch_cols_any<T>(c, wk, nb, 1, false, false, ka))) return rc;
+      if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, ka))) return rc;
+      if ((rc = launch_cols_any<T>(c, wk, nb, 1, true, false, ka))) return rc;
       if ((rc = launch_x_any<T>(c, wk, co, nb, true, 1, ci, pot, (T)a, (T)b))) return rc;
     }
   }
@@ -756,8 +818,9 @@ int forward_fft64(fbse_ctx *c, double2 *data, double2 *work)
 {
   int rc;
   if ((rc = launch_x<double>(c, data, work, 1, false, 0, nullptr, nullptr, 1.0, 0.0))) return rc;
-  if ((rc = launch_cols<double>(c, work, 1, 1, false, false))) return rc;
-  if ((rc = launch_cols<double>(c, work, 1, 2, false, false))) return rc;
+  const KinArgs ka = kin_args(c, nullptr, false, false);
+  if ((rc = launch_cols<double>(c, work, 1, 1, false, false, ka))) return rc;
+  if ((rc = launch_cols<double>(c, work, 1, 2, false, false, ka))) return rc;
   FBSE_CUDA(c, cudaMemcpyAsync(data, work, c->ngrid * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
   return FBSE_OK;
 }

@@ -66,7 +66,15 @@ struct KinArgs {
   double kemax;
   const double2 *kq;  // when set: multiply by this complex k-space array instead
   long nx, nxy;
+  const int *ordx, *ordy;  // k index of an x / y position where that axis is not in k order (the k2 tables
+                           // above are in the positions' order already)
 };
+
+// offset in a k-space plane of the point at positions (x, y)
+__device__ __forceinline__ long kin_xy(const KinArgs &ka, int x, int y)
+{
+  return (long)(ka.ordy ? ka.ordy[y] : y) * ka.nx + (ka.ordx ? ka.ordx[x] : x);
+}
 
 // min(0.5 k^2, KE_max) / N from the per-axis tables, in the working precision
 template <typename T> __device__ __forceinline__ T kin_factor(const KinArgs &ka, int x, int y, int z);
@@ -81,5 +89,16 @@ template <> __device__ __forceinline__ float kin_factor<float>(const KinArgs &ka
   const float cap = (float)ka.kemax;
   return kk > cap ? cap : kk;
 }
+
+// two-factor kernels (fft_two.cuh): one xy plane per CTA, the z pass, and the
+// y and x line passes for planes larger than shared memory.  x and y transforms
+// leave k = k1 + Q k2 at position k2 + P k1 (AxisPlan::ord)
+template <typename T> size_t two_plane_smem(const fbse_ctx *c);
+template <typename T>
+int two_plane(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T> *phi, const T *pot, T ca, T cb);
+template <typename T> int two_z(fbse_ctx *c, C<T> *data, long nblk, const KinArgs &ka);
+template <typename T> int two_y(fbse_ctx *c, C<T> *data, long nblk, bool inv);
+template <typename T>
+int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T> *phi, const T *pot, T ca, T cb);
 
 }  // namespace fbse

@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(ColsCfg<T, N>::THREADS, ColsCfg<T, N>::MINB)
         const int k = t + P * j + Q * k2;
         if (ka.kq) {
           // convolution: multiply by the k-space array (hartree, bse_cplx/hartree.c:19-27)
-          const double2 q = ka.kq[(long)k * ka.nxy + (long)jy * ka.nx + x];
+          const double2 q = ka.kq[(long)k * ka.nxy + kin_xy(ka, x, jy)];
           v[j * P + k2] = cmul<T>(v[j * P + k2], mk<T>((T)q.x, (T)q.y));
         } else {
           v[j * P + k2] = cscale<T>(v[j * P + k2], kin_factor<T>(ka, x, jy, k));

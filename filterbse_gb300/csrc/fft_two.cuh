@@ -1,0 +1,449 @@
+// Two-factor FFT kernels for axis lengths n = P Q (P <= Q, both radices that a
+// thread transforms in registers, fft_radix.cuh): every length up to 16 x 16
+// whose factors allow it, and lengths with one radix of 17 .. 31.
+//
+// Decomposition (input n = t + P m, output k = k1 + Q k2):
+//   X[k1 + Q k2] = sum_t w_P^{t k2} [ w_n^{t k1} sum_m x[t + P m] w_Q^{m k1} ]
+// Stage A transforms the Q values at positions t + P m and leaves Y_t[k1],
+// already times w_n^{t k1}, at positions t + P k1; stage B transforms the P
+// values at positions P k1 .. P k1 + P - 1.  Both stages are in place, and the
+// twiddle of position p is tw[p] in both directions.  The result for k = k1 + Q k2
+// stays at position k2 + P k1: every pass between the forward and the inverse
+// transform of an axis is pointwise in that axis, so x and y keep this order
+// (AxisPlan::ord maps a position to its k, AxisPlan::k2o is the kinetic table in
+// it) and no pass reorders.  The inverse runs the stages backwards (B with the
+// twiddles, then A), as a forward transform of exchanged real and imaginary parts.
+//
+// A stage's work items are (butterfly, line) pairs with the line fastest, so the
+// lanes of a warp take consecutive lines (one broadcast twiddle, coalesced or
+// conflict-free accesses) and no lane idles when the line count is not a
+// multiple of 32.
+//
+// Why: the one-radix-per-pass Stockham kernels (fft.cu) spend 3-4 shared-memory
+// round trips and an integer division per element on such lengths, and lengths
+// with a prime above 8 take a direct sum per output.  Measured, H psi through
+// those kernels -> these:
+//   116 x 117 x 120, 4 spinors, FP32 (memory and latency bound)  2101 -> 408 us
+//   96^3, 4 spinors, FP32 (127 terms of a filter)                  742 -> 214 us
+//   96^3, 6 spinors, FP64 (FP64 pipe bound; projectors 1.9 ms)     5131 -> 3921 us
+//   57 x 52 x 45, 8 packed states, FP64 (radices 13, 19)           1911 -> 513 us
+#pragma once
+
+#include <type_traits>
+
+#include "fft_radix.cuh"
+
+namespace fbse {
+namespace two {
+
+// x / d for x * d < 2^32
+struct Div {
+  unsigned d, m;
+  __host__ __device__ explicit Div(unsigned d_ = 1) : d(d_), m((unsigned)(0xffffffffu / d_) + 1u) {}
+  __device__ __forceinline__ unsigned operator()(unsigned x) const { return d == 1 ? x : __umulhi(x, m); }
+};
+
+template <typename T> struct Axis {
+  int n, P, Q;
+  const C<T> *tw;  // tw[t + P k1] = w_n^{t k1}
+};
+
+// calls f(integral_constant<R>) for the run-time radix r.  BIG: the set with the
+// radices above 16
+template <bool BIG, typename F> __device__ __forceinline__ void with_radix(int r, F f)
+{
+#define FBSE_R(R) \
+  case R: f(std::integral_constant<int, R>{}); break;
+  switch (r) {
+    FBSE_R(1) FBSE_R(2) FBSE_R(3) FBSE_R(4) FBSE_R(5) FBSE_R(6) FBSE_R(7) FBSE_R(8) FBSE_R(9) FBSE_R(10) FBSE_R(11)
+    FBSE_R(12) FBSE_R(13) FBSE_R(14) FBSE_R(15) FBSE_R(16)
+    default:
+      if constexpr (BIG) {
+        switch (r) {
+          FBSE_R(17) FBSE_R(18) FBSE_R(19) FBSE_R(20) FBSE_R(21) FBSE_R(23) FBSE_R(24) FBSE_R(25) FBSE_R(29)
+          FBSE_R(31)
+        }
+      }
+  }
+#undef FBSE_R
+}
+
+template <typename T> __device__ __forceinline__ C<T> exch(C<T> v) { return mk<T>(v.y, v.x); }
+
+// one stage over L lines: butterflies j < nb at positions first(j) + step i,
+// i < R.  ld(line, position) and st(line, position, value); TW: multiply by
+// tw[position] before the store
+template <typename T, bool BIG, bool TW, typename Ld, typename St>
+__device__ __forceinline__ void stage(int R, int nb, int mul, int step, const Div &lines, const C<T> *__restrict__ tw,
+                                      Ld ld, St st)
+{
+  with_radix<BIG>(R, [&](auto rc) {
+    constexpr int RR = decltype(rc)::value;
+    const unsigned items = (unsigned)nb * lines.d;
+    for (unsigned it = threadIdx.x; it < items; it += blockDim.x) {
+      const unsigned j = lines(it);
+      const int c = (int)(it - j * lines.d), p0 = (int)j * mul;
+      C<T> v[RR];
+#pragma unroll
+      for (int i = 0; i < RR; i++) v[i] = ld(c, p0 + i * step);
+      dft<T, RR>(v);
+#pragma unroll
+      for (int i = 0; i < RR; i++) {
+        if (TW && i > 0) v[i] = cmul<T>(v[i], __ldg(tw + p0 + i * step));
+        st(c, p0 + i * step, v[i]);
+      }
+    }
+  });
+}
+// stage A: P butterflies of Q values; stage B: Q butterflies of P values
+template <typename T, bool BIG, bool TW, typename Ld, typename St>
+__device__ __forceinline__ void stage_a(const Axis<T> &a, const Div &lines, Ld ld, St st)
+{
+  stage<T, BIG, TW>(a.Q, a.P, 1, a.P, lines, a.tw, ld, st);
+}
+template <typename T, bool TW, typename Ld, typename St>
+__device__ __forceinline__ void stage_b(const Axis<T> &a, const Div &lines, Ld ld, St st)
+{
+  stage<T, false, TW>(a.P, a.Q, a.P, 1, lines, a.tw, ld, st);
+}
+
+__device__ __forceinline__ void copy_async(float2 *dst, const float2 *src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void copy_async(double2 *dst, const double2 *src)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// out = ca (r + V phi) + cb phi
+template <typename T>
+__device__ __forceinline__ C<T> epilogue(C<T> r, C<T> ph, const T *__restrict__ pot, long g, T ca, T cb)
+{
+  if (pot) {
+    const T V = pot[g];
+    r.x += V * ph.x;
+    r.y += V * ph.y;
+  }
+  return mk<T>(ca * r.x + cb * ph.x, ca * r.y + cb * ph.y);
+}
+
+// ---------------------------------------------------------------------------
+// plane pass: one xy plane per CTA in shared memory (row stride nx | 1: lanes on
+// consecutive x or consecutive y are free of bank conflicts).
+//   INV false: y forward (its first stage reads the plane from global memory,
+//   lanes along x), x forward, store
+//   INV true: load, x inverse, y inverse; the last y stage holds final values
+//   with lanes along x and writes out = ca (r + V phi) + cb phi itself
+// Registers: 64 (FP32, up to 1024 threads a CTA) / 128 (FP64, up to 512) keep two
+// or more CTAs of a 100 x 100 plane on an SM, whose phases then overlap.
+// ---------------------------------------------------------------------------
+template <typename T, bool BIG> struct PlaneShape {
+  static constexpr int threads = (sizeof(T) == 4 ? 1024 : 512) / (BIG ? 2 : 1);
+};
+
+template <typename T, bool BIG, bool INV>
+__global__ void __launch_bounds__(PlaneShape<T, BIG>::threads, 1)
+    k_two_plane(const C<T> *__restrict__ in, C<T> *__restrict__ out, Axis<T> ax, Axis<T> ay, Div dx, Div dy,
+                const C<T> *__restrict__ phi, const T *__restrict__ pot, long ngrid, T ca, T cb)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C<T> *S = reinterpret_cast<C<T> *>(smem_raw);
+  const int nx = ax.n, pitch = nx | 1;
+  const unsigned npl = (unsigned)nx * ay.n;
+  const long base = (long)blockIdx.x * npl;
+  auto ycol = [&](int x, int y) -> C<T> & { return S[y * pitch + x]; };
+  auto xrow = [&](int y, int x) -> C<T> & { return S[y * pitch + x]; };
+  auto ldy = [&](int x, int y) { return ycol(x, y); };
+  auto sty = [&](int x, int y, C<T> v) { ycol(x, y) = v; };
+  auto ldx = [&](int y, int x) { return xrow(y, x); };
+  auto stx = [&](int y, int x, C<T> v) { xrow(y, x) = v; };
+  if constexpr (!INV) {
+    const C<T> *src = in + base;
+    stage_a<T, BIG, true>(ay, dx, [&](int x, int y) { return src[y * nx + x]; }, sty);
+    __syncthreads();
+    stage_b<T, false>(ay, dx, ldy, sty);
+    __syncthreads();
+    stage_a<T, BIG, true>(ax, dy, ldx, stx);
+    __syncthreads();
+    stage_b<T, false>(ax, dy, ldx, stx);
+    __syncthreads();
+    C<T> *dst = out + base;
+#pragma unroll 4
+    for (unsigned i = threadIdx.x; i < npl; i += blockDim.x) {
+      const unsigned y = dx(i);
+      dst[i] = S[i + y * (pitch - nx)];
+    }
+  } else {
+    const C<T> *src = in + base;
+    for (unsigned i = threadIdx.x; i < npl; i += blockDim.x) {
+      const unsigned y = dx(i);
+      copy_async(S + i + y * (pitch - nx), src + i);
+    }
+    copy_wait();
+    __syncthreads();
+    stage_b<T, true>(ax, dy, [&](int y, int x) { return exch<T>(xrow(y, x)); }, stx);
+    __syncthreads();
+    stage_a<T, BIG, false>(ax, dy, ldx, stx);
+    __syncthreads();
+    stage_b<T, true>(ay, dx, ldy, sty);
+    __syncthreads();
+    const C<T> *ph = phi + base;
+    const T *V = pot ? pot + base % ngrid : nullptr;
+    C<T> *dst = out + base;
+    stage_a<T, BIG, false>(ay, dx, ldy, [&](int x, int y, C<T> v) {
+      const int o = y * nx + x;
+      dst[o] = epilogue<T>(exch<T>(v), ph[o], V, o, ca, cb);
+    });
+  }
+}
+
+// ---------------------------------------------------------------------------
+// line kernels: tiles of up to L lines in shared memory
+// ---------------------------------------------------------------------------
+template <typename T, bool BIG> struct LineShape {
+  static constexpr int threads = BIG ? 256 : 512;
+  static constexpr int ctas = sizeof(T) == 4 ? 2 : 1;
+};
+
+// z: forward, times the kinetic factor (or the k-space array ka.kq), inverse.
+// A tile is L consecutive points of the flattened xy plane, whatever nx is.
+template <typename T, bool BIG>
+__global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>::ctas)
+    k_two_z(C<T> *__restrict__ data, Axis<T> az, int L, int ntile, long ngrid, KinArgs ka)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C<T> *S = reinterpret_cast<C<T> *>(smem_raw);
+  const long blk = blockIdx.x / ntile;
+  const int c0 = (int)(blockIdx.x - blk * ntile) * L;
+  const int nl = min(L, (int)ka.nxy - c0);
+  const Div lines((unsigned)nl);
+  const long es = ka.nxy;
+  C<T> *d = data + blk * ngrid + c0;
+  auto lds = [&](int c, int z) { return S[z * L + c]; };
+  auto sts = [&](int c, int z, C<T> v) { S[z * L + c] = v; };
+  stage_a<T, BIG, true>(az, lines, [&](int c, int z) { return d[z * es + c]; }, sts);
+  __syncthreads();
+  with_radix<false>(az.P, [&](auto rc) {
+    constexpr int RR = decltype(rc)::value;
+    const unsigned items = (unsigned)(az.Q * nl);
+    for (unsigned it = threadIdx.x; it < items; it += blockDim.x) {
+      const unsigned k1 = lines(it);
+      const int c = (int)(it - k1 * nl);
+      C<T> *s = S + (int)k1 * RR * L + c;
+      C<T> v[RR];
+#pragma unroll
+      for (int i = 0; i < RR; i++) v[i] = s[i * L];
+      dft<T, RR>(v);
+      const int g = c0 + c, y = g / (int)ka.nx, x = g - y * (int)ka.nx;
+      if (ka.kq) {
+        const double2 *q = ka.kq + kin_xy(ka, x, y);
+#pragma unroll
+        for (int i = 0; i < RR; i++) {
+          const double2 w = q[(long)((int)k1 + az.Q * i) * es];
+          v[i] = cmul<T>(v[i], mk<T>((T)w.x, (T)w.y));
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < RR; i++) v[i] = cscale<T>(v[i], kin_factor<T>(ka, x, y, (int)k1 + az.Q * i));
+      }
+#pragma unroll
+      for (int i = 0; i < RR; i++) v[i] = exch<T>(v[i]);
+      dft<T, RR>(v);
+#pragma unroll
+      for (int i = 0; i < RR; i++) {
+        if (i > 0) v[i] = cmul<T>(v[i], __ldg(az.tw + (int)k1 * RR + i));
+        s[i * L] = v[i];
+      }
+    }
+  });
+  __syncthreads();
+  stage_a<T, BIG, false>(az, lines, lds, [&](int c, int z, C<T> v) { d[z * es + c] = exch<T>(v); });
+}
+
+// y lines of planes too large for shared memory: L consecutive x of one plane,
+// global memory to global memory, one exchange
+template <typename T, bool BIG, bool INV>
+__global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>::ctas)
+    k_two_y(C<T> *__restrict__ data, Axis<T> ay, int nx, int L, int ntile)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C<T> *S = reinterpret_cast<C<T> *>(smem_raw);
+  const long pl = blockIdx.x / ntile;
+  const int x0 = (int)(blockIdx.x - pl * ntile) * L;
+  const Div lines((unsigned)min(L, nx - x0));
+  C<T> *d = data + pl * nx * ay.n + x0;
+  auto ldg = [&](int c, int y) { return INV ? exch<T>(d[y * nx + c]) : d[y * nx + c]; };
+  auto stg = [&](int c, int y, C<T> v) { d[y * nx + c] = INV ? exch<T>(v) : v; };
+  auto lds = [&](int c, int y) { return S[y * L + c]; };
+  auto sts = [&](int c, int y, C<T> v) { S[y * L + c] = v; };
+  if constexpr (!INV) {
+    stage_a<T, BIG, true>(ay, lines, ldg, sts);
+    __syncthreads();
+    stage_b<T, false>(ay, lines, lds, stg);
+  } else {
+    stage_b<T, true>(ay, lines, ldg, sts);
+    __syncthreads();
+    stage_a<T, BIG, false>(ay, lines, lds, stg);
+  }
+}
+
+// x lines: L contiguous lines through shared memory with an odd line stride
+// (coalesced copies, lanes on consecutive lines in the stages); INV ends with
+// out = ca (r + V phi) + cb phi
+template <typename T, bool BIG, bool INV>
+__global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>::ctas)
+    k_two_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Axis<T> ax, Div dn, long nlines, int L,
+            const C<T> *__restrict__ phi, const T *__restrict__ pot, long ngrid, T ca, T cb)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C<T> *S = reinterpret_cast<C<T> *>(smem_raw);
+  const int n = ax.n, pitch = n | 1;
+  const long l0 = (long)blockIdx.x * L;
+  const Div lines((unsigned)min((long)L, nlines - l0));
+  const unsigned count = lines.d * n;
+  const long off = l0 * n;
+  const C<T> *src = in + off;
+  for (unsigned i = threadIdx.x; i < count; i += blockDim.x) copy_async(S + i + dn(i) * (pitch - n), src + i);
+  copy_wait();
+  __syncthreads();
+  auto ldx = [&](int y, int x) { return S[y * pitch + x]; };
+  auto stx = [&](int y, int x, C<T> v) { S[y * pitch + x] = v; };
+  C<T> *dst = out + off;
+  if constexpr (!INV) {
+    stage_a<T, BIG, true>(ax, lines, ldx, stx);
+    __syncthreads();
+    stage_b<T, false>(ax, lines, ldx, stx);
+    __syncthreads();
+#pragma unroll 4
+    for (unsigned i = threadIdx.x; i < count; i += blockDim.x) dst[i] = S[i + dn(i) * (pitch - n)];
+  } else {
+    stage_b<T, true>(ax, lines, [&](int y, int x) { return exch<T>(S[y * pitch + x]); }, stx);
+    __syncthreads();
+    stage_a<T, BIG, false>(ax, lines, ldx, stx);
+    __syncthreads();
+#pragma unroll 4
+    for (unsigned i = threadIdx.x; i < count; i += blockDim.x) {
+      const C<T> r = exch<T>(S[i + dn(i) * (pitch - n)]);
+      long g = off + i;  // the lines of a tile may lie in two blocks
+      dst[i] = epilogue<T>(r, phi[g], pot, pot ? g % ngrid : 0, ca, cb);
+    }
+  }
+}
+
+}  // namespace two
+}  // namespace fbse
+
+// ---------------------------------------------------------------------------
+// launches
+// ---------------------------------------------------------------------------
+namespace fbse {
+namespace two {
+
+template <typename T> static Axis<T> axis_of(const AxisPlan &p)
+{
+  if constexpr (sizeof(T) == 4) return {p.n, p.P, p.Q, p.two32};
+  else return {p.n, p.P, p.Q, p.two64};
+}
+
+template <typename K, typename... Args>
+static int launch(fbse_ctx *c, K kernel, long grid, int threads, size_t smem, Args... args)
+{
+  if (grid > 2147483647L) return set_err(c, FBSE_ERR_UNSUPPORTED, "FFT batch too large for one launch");
+  FBSE_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<(unsigned)grid, threads, smem, c->stream>>>(args...);
+  FBSE_CHECK_LAUNCH(c);
+  return FBSE_OK;
+}
+
+inline int round32(long v, int lo, int hi)
+{
+  const long r = (v + 31) / 32 * 32;
+  return (int)(r < lo ? lo : r > hi ? hi : r);
+}
+
+// threads of a plane CTA: the register file's share when as many CTAs as fit
+// (shared memory, or the planes there are) sit on each SM
+template <typename T, bool BIG> static int plane_threads(fbse_ctx *c, size_t smem, long grid)
+{
+  const long fit = std::max<long>(1, std::min<long>((long)(228 * 1024 / (smem + 1024)), (grid + 151) / 152));
+  const long work = std::max(c->ax[0].P * c->ny, c->ax[1].P * c->nx);
+  return round32(std::min<long>(work, PlaneShape<T, BIG>::threads / fit), 128, PlaneShape<T, BIG>::threads);
+}
+
+// lines per tile: 256-byte segments, half of that when a launch would leave SMs idle
+template <typename T> static int tile_lines(long lines, long groups)
+{
+  const int full = 256 / (int)sizeof(C<T>);
+  int L = groups * ((lines + full - 1) / full) < 304 ? full / 2 : full;
+  const long nt = (lines + L - 1) / L;
+  return (int)((lines + nt - 1) / nt);  // even tiles
+}
+
+}  // namespace two
+
+template <typename T> size_t two_plane_smem(const fbse_ctx *c) { return (size_t)(c->nx | 1) * c->ny * sizeof(C<T>); }
+
+template <typename T>
+int two_plane(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T> *phi, const T *pot, T ca, T cb)
+{
+  using namespace two;
+  const size_t smem = two_plane_smem<T>(c);
+  const long grid = nblk * c->nz;
+  const Axis<T> ax = axis_of<T>(c->ax[0]), ay = axis_of<T>(c->ax[1]);
+  const Div dx((unsigned)c->nx), dy((unsigned)c->ny);
+  const bool big = ax.Q > 16 || ay.Q > 16;
+  const int th = big ? plane_threads<T, true>(c, smem, grid) : plane_threads<T, false>(c, smem, grid);
+  auto go = [&](auto k) { return launch(c, k, grid, th, smem, in, out, ax, ay, dx, dy, phi, pot, c->ngrid, ca, cb); };
+  if (big) return inv ? go(k_two_plane<T, true, true>) : go(k_two_plane<T, true, false>);
+  return inv ? go(k_two_plane<T, false, true>) : go(k_two_plane<T, false, false>);
+}
+
+template <typename T> int two_z(fbse_ctx *c, C<T> *data, long nblk, const KinArgs &ka)
+{
+  using namespace two;
+  const Axis<T> az = axis_of<T>(c->ax[2]);
+  const int L = tile_lines<T>(ka.nxy, nblk);
+  const int ntile = (int)((ka.nxy + L - 1) / L);
+  const size_t smem = (size_t)az.n * L * sizeof(C<T>);
+  if (az.Q > 16)
+    return launch(c, k_two_z<T, true>, nblk * ntile, round32((long)az.P * L, 64, LineShape<T, true>::threads), smem,
+                  data, az, L, ntile, c->ngrid, ka);
+  return launch(c, k_two_z<T, false>, nblk * ntile, round32((long)az.P * L, 64, LineShape<T, false>::threads), smem,
+                data, az, L, ntile, c->ngrid, ka);
+}
+
+template <typename T> int two_y(fbse_ctx *c, C<T> *data, long nblk, bool inv)
+{
+  using namespace two;
+  const Axis<T> ay = axis_of<T>(c->ax[1]);
+  const int L = tile_lines<T>(c->nx, nblk * c->nz);
+  const int ntile = (int)((c->nx + L - 1) / L);
+  const size_t smem = (size_t)ay.n * L * sizeof(C<T>);
+  const bool big = ay.Q > 16;
+  const int th = round32((long)ay.P * L, 64, big ? LineShape<T, true>::threads : LineShape<T, false>::threads);
+  auto go = [&](auto k) { return launch(c, k, nblk * c->nz * ntile, th, smem, data, ay, (int)c->nx, L, ntile); };
+  if (big) return inv ? go(k_two_y<T, true, true>) : go(k_two_y<T, true, false>);
+  return inv ? go(k_two_y<T, false, true>) : go(k_two_y<T, false, false>);
+}
+
+template <typename T>
+int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T> *phi, const T *pot, T ca, T cb)
+{
+  using namespace two;
+  const Axis<T> ax = axis_of<T>(c->ax[0]);
+  const long nlines = nblk * c->ny * c->nz;
+  const int L = tile_lines<T>(nlines, 1);
+  const size_t smem = (size_t)(ax.n | 1) * L * sizeof(C<T>);
+  const Div dn((unsigned)ax.n);
+  const bool big = ax.Q > 16;
+  const int th = round32((long)ax.P * L, 64, big ? LineShape<T, true>::threads : LineShape<T, false>::threads);
+  auto go = [&](auto k) {
+    return launch(c, k, (nlines + L - 1) / L, th, smem, in, out, ax, dn, nlines, L, phi, pot, c->ngrid, ca, cb);
+  };
+  if (big) return inv ? go(k_two_x<T, true, true>) : go(k_two_x<T, true, false>);
+  return inv ? go(k_two_x<T, false, true>) : go(k_two_x<T, false, false>);
+}
+
+}  // namespace fbse

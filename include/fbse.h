@@ -116,8 +116,8 @@ void *fbse_stream(fbse_ctx *ctx);
  * nonzero field fixes the choice.  Set it before the first compute call; the
  * first call of each batch size should come before any stream capture. */
 typedef struct fbse_tuning {
-  int fft_kernels;         /* 0: register-resident kernels for 64/128/256-point axes where they fit,
-                              mixed-radix elsewhere; 1: mixed-radix kernels on every axis; 2: mixed-radix
+  int fft_kernels;         /* 0: register-resident kernels for 64/128/256-point axes where they fit, two-factor
+                              kernels for lengths with two register radices, mixed-radix elsewhere; 1: mixed-radix kernels on every axis; 2: mixed-radix
                               x lines and y/z columns (no plane kernel).  Results differ in rounding only */
   int fft_plane_cluster;   /* 0: one CTA per 128 x 128 FP32 plane; 1: two-CTA clusters (same results) */
   long fft_chunk_blocks;   /* 3D blocks (state x spin) per FFT launch sequence; 0: autotuned */
