@@ -63,6 +63,8 @@ struct AxisPlan {
   int P = 0, Q = 0;
   double2 *two64 = nullptr;
   float2 *two32 = nullptr;
+  double2 *sym64 = nullptr;  // (cos, sin)(2 pi q r / Q) of fft_two.cuh's stage_sym, for the Q it takes
+  float2 *sym32 = nullptr;
   int *ord = nullptr;
   double *k2o = nullptr;
   float *k2of = nullptr;
@@ -152,6 +154,9 @@ struct fbse_ctx {
   double *red = nullptr; size_t red_bytes = 0;   // reduction partials
   int *dstatus = nullptr;                        // device error flags of kernels with bounded waits
   int tc_poisoned = 0;  // a tensor-core wait timed out: MMAs may still be in flight, the path is refused
+  // the FP32 Rayleigh-Ritz step (ortho_diag_sigma) is running: H psi takes the
+  // mixed-radix FFT kernels on every axis that the register-resident ones do not
+  int steady = 0;
   int nsm = 0;          // multiprocessors of the device (queried on first use)
   // large buffers kept between calls (grown on demand, freed by fbse_destroy):
   // the Newton ring, the Rayleigh-Ritz H psi and rotated states, the

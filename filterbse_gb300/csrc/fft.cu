@@ -65,16 +65,19 @@ static std::vector<int> factorize(int n)
 }
 
 // n = P Q for the two-factor kernels: both radices at most 16 and as close as
-// possible, else the largest P with a Q of the second set; false: neither
+// possible, else the largest P with a register radix up to 31, else with an
+// odd Q up to kSymMax (stage_sym); false: none of them
+constexpr int kSymMin = 27, kSymMax = 255;
 static bool two_factors(int n, int *P, int *Q)
 {
-  for (int set = 0; set < 2; set++)
+  for (int set = 0; set < 3; set++)
     for (int p = 16; p >= 1; p--) {
       const int q = n / p;
       if (n % p || q < p) continue;
       const bool second = q == 17 || q == 18 || q == 19 || q == 20 || q == 21 || q == 23 || q == 24 || q == 25 ||
                           q == 29 || q == 31;
-      if (set == 0 ? q <= 16 : second) {
+      const bool third = q % 2 == 1 && q >= kSymMin && q <= kSymMax;
+      if (set == 0 ? q <= 16 : set == 1 ? second : third) {
         *P = p;
         *Q = q;
         return true;
@@ -117,12 +120,28 @@ int plan_axis(fbse_ctx *c, AxisPlan &p, int n)
     FBSE_CUDA(c, cudaMemcpy(p.two64, t64.data(), n * sizeof(double2), cudaMemcpyHostToDevice));
     FBSE_CUDA(c, cudaMemcpy(p.two32, t32.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
   }
+  if (p.P > 0 && p.Q >= kSymMin && p.Q != 29 && p.Q != 31) {
+    // stage_sym's coefficients [r - 1][row block][row], rows beyond Q / 2 zero
+    const int h = p.Q / 2, rows = (h + kSymRows) / kSymRows * kSymRows;
+    std::vector<double2> s64((size_t)h * rows, make_double2(0, 0));
+    std::vector<float2> s32((size_t)h * rows, make_float2(0, 0));
+    for (int r = 1; r <= h; r++)
+      for (int q = 0; q <= h; q++) {
+        const double2 w = h64[(long)q * r % p.Q * (n / p.Q)];
+        s64[(size_t)(r - 1) * rows + q] = make_double2(w.x, -w.y);
+        s32[(size_t)(r - 1) * rows + q] = make_float2((float)w.x, (float)-w.y);
+      }
+    FBSE_CUDA(c, cudaMalloc(&p.sym64, s64.size() * sizeof(double2)));
+    FBSE_CUDA(c, cudaMalloc(&p.sym32, s32.size() * sizeof(float2)));
+    FBSE_CUDA(c, cudaMemcpy(p.sym64, s64.data(), s64.size() * sizeof(double2), cudaMemcpyHostToDevice));
+    FBSE_CUDA(c, cudaMemcpy(p.sym32, s32.data(), s32.size() * sizeof(float2), cudaMemcpyHostToDevice));
+  }
   return FBSE_OK;
 }
 
 void free_axis(AxisPlan &p)
 {
-  void *bufs[] = {p.tw64, p.tw32, p.two64, p.two32, p.ord, p.k2o, p.k2of};
+  void *bufs[] = {p.tw64, p.tw32, p.two64, p.two32, p.sym64, p.sym32, p.ord, p.k2o, p.k2of};
   for (void *b : bufs)
     if (b) cudaFree(b);
   p = AxisPlan();
@@ -670,7 +689,7 @@ static int launch_cols_fast_n(fbse_ctx *c, C<T> *data, long nblk, int axis, bool
 // two-factor kernels (fft_two.cuh): any other length that has the two factors
 static bool two_axis_ok(fbse_ctx *c, int axis)
 {
-  return c->tune.fft_kernels == 0 && c->ax[axis].P > 0 && !fast_axis_ok(c, c->ax[axis].n);
+  return c->tune.fft_kernels == 0 && !c->steady && c->ax[axis].P > 0 && !fast_axis_ok(c, c->ax[axis].n);
 }
 
 // y or z lines; z (kmul): forward, multiply, inverse
@@ -738,7 +757,7 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
   const T *pot = with_v ? pot_of<T>(c) : nullptr;
   const bool fplane = fast_plane_ok<T>(c);
   // a plane of two lengths that both have two factors (64, 128 and 256 do) when it fits
-  const bool tplane = !fplane && c->tune.fft_kernels == 0 && c->ax[0].P > 0 && c->ax[1].P > 0 &&
+  const bool tplane = !fplane && c->tune.fft_kernels == 0 && !c->steady && c->ax[0].P > 0 && c->ax[1].P > 0 &&
                       two_plane_smem<T>(c) <= (size_t)max_smem();
   const bool lines = two_axis_ok(c, 0) || two_axis_ok(c, 1);
   const bool plane = !lines && !sx.big && !sy.big && plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;

@@ -90,6 +90,9 @@ template <> __device__ __forceinline__ float kin_factor<float>(const KinArgs &ka
   return kk > cap ? cap : kk;
 }
 
+// rows a thread of fft_two.cuh's stage_sym sums
+constexpr int kSymRows = 8;
+
 // two-factor kernels (fft_two.cuh): one xy plane per CTA, the z pass, and the
 // y and x line passes for planes larger than shared memory.  x and y transforms
 // leave k = k1 + Q k2 at position k2 + P k1 (AxisPlan::ord)

@@ -1,6 +1,7 @@
-// Two-factor FFT kernels for axis lengths n = P Q (P <= Q, both radices that a
-// thread transforms in registers, fft_radix.cuh): every length up to 16 x 16
-// whose factors allow it, and lengths with one radix of 17 .. 31.
+// Two-factor FFT kernels for axis lengths n = P Q, P <= Q, P <= 16 a radix that a
+// thread transforms in registers (fft_radix.cuh) and Q one such radix up to 31,
+// or any odd number of 27 .. 255 (stage_sym): the reference's grid rule gives
+// every even length, so factors 2 x 43 or 4 x 37 are as common as smooth ones.
 //
 // Decomposition (input n = t + P m, output k = k1 + Q k2):
 //   X[k1 + Q k2] = sum_t w_P^{t k2} [ w_n^{t k1} sum_m x[t + P m] w_Q^{m k1} ]
@@ -45,11 +46,12 @@ struct Div {
 
 template <typename T> struct Axis {
   int n, P, Q;
-  const C<T> *tw;  // tw[t + P k1] = w_n^{t k1}
+  const C<T> *tw;   // tw[t + P k1] = w_n^{t k1}
+  const C<T> *sym;  // stage_sym's coefficients when Q is transformed there, else null
 };
 
 // calls f(integral_constant<R>) for the run-time radix r.  BIG: the set with the
-// radices above 16
+// radices above 16 (kernels with BIG also hold stage_sym)
 template <bool BIG, typename F> __device__ __forceinline__ void with_radix(int r, F f)
 {
 #define FBSE_R(R) \
@@ -95,10 +97,135 @@ __device__ __forceinline__ void stage(int R, int nb, int mul, int step, const Di
     }
   });
 }
-// stage A: P butterflies of Q values; stage B: Q butterflies of P values
-template <typename T, bool BIG, bool TW, typename Ld, typename St>
-__device__ __forceinline__ void stage_a(const Axis<T> &a, const Div &lines, Ld ld, St st)
+// stage A for an odd Q too large for a thread's registers: P butterflies of Q
+// values, each shared by the threads of its row blocks.  With a_r = x_r + x_{Q-r}
+// and b_r = x_r - x_{Q-r} (formed in place first), row q of the block sums
+// e_q = x_0 + sum_r cos a_r and o_q = sum_r sin b_r, which give X_q and X_{Q-q}:
+// Q multiply-adds per value, the quarter of a direct sum.  kSymRows rows per
+// thread share each a_r, b_r, and kSymLines lines share each coefficient (FP32,
+// where the loads and not the FP32 pipe bound the sums); the lanes of a warp take
+// consecutive lines, so the coefficients are broadcasts.  A group of lines keeps
+// its sums in registers until every thread has read the group's values, so the
+// stage is in place.
+// H psi without projectors, FP32, 8 states: 86^3 307 us, 118^3 800 us (the loads of
+// the coefficients bound it: two lines a thread measured 342 and 861 us with one,
+// and 362 and 939 us with the next coefficients fetched ahead); FP64, 4 states of
+// 86^3: 2212 us, 60% of the FP64 pipe.  The direct sums took 4 times as long.
+template <typename T> constexpr int kSymLines = sizeof(T) == 4 ? 2 : 1;
+
+// a row block's coefficients of one r, 16 bytes a load
+__device__ __forceinline__ void ld_coef(const float2 *w, float2 (&cs)[kSymRows])
 {
+  const float4 *v = reinterpret_cast<const float4 *>(w);
+#pragma unroll
+  for (int i = 0; i < kSymRows / 2; i++) {
+    const float4 q = __ldg(v + i);
+    cs[2 * i] = make_float2(q.x, q.y);
+    cs[2 * i + 1] = make_float2(q.z, q.w);
+  }
+}
+__device__ __forceinline__ void ld_coef(const double2 *w, double2 (&cs)[kSymRows])
+{
+#pragma unroll
+  for (int i = 0; i < kSymRows; i++) cs[i] = __ldg(w + i);
+}
+
+template <typename T, bool TW, typename Ld, typename At, typename St>
+__device__ __forceinline__ void stage_sym(const Axis<T> &a, const Div &lines, Ld ld, At at, St st)
+{
+  const int P = a.P, Q = a.Q, H = Q >> 1, nqb = (H + kSymRows) / kSymRows, L = (int)lines.d;
+  const Div dp((unsigned)P);
+  for (unsigned it = threadIdx.x; it < (unsigned)((H + 1) * P * L); it += blockDim.x) {
+    const unsigned j = lines(it), r = dp(j);
+    const int c = (int)(it - j * L), t = (int)(j - r * P);
+    const C<T> x = ld(c, t + P * (int)r);
+    if (r == 0) {
+      at(c, t) = x;
+    } else {
+      const C<T> y = ld(c, t + P * (Q - (int)r));
+      at(c, t + P * (int)r) = cadd<T>(x, y);
+      at(c, t + P * (Q - (int)r)) = csub<T>(x, y);
+    }
+  }
+  __syncthreads();
+  // a thread's lines: c and c + half of its group
+  const int per = P * nqb, Lg = kSymLines<T> * ((int)blockDim.x / per);  // the launch gives at least per threads
+  for (int l0 = 0; l0 < L; l0 += Lg) {
+    const int nl = min(Lg, L - l0), half = (nl + kSymLines<T> - 1) / kSymLines<T>;
+    const int j = (int)threadIdx.x / half, k = (int)threadIdx.x % half;
+    const int qb = (int)dp((unsigned)j), t = j - qb * P;
+    int c[kSymLines<T>];
+    bool act[kSymLines<T>];
+#pragma unroll
+    for (int u = 0; u < kSymLines<T>; u++) {
+      act[u] = j < per && k + u * half < nl;
+      c[u] = l0 + (act[u] ? k + u * half : k);
+    }
+    C<T> e[kSymLines<T>][kSymRows], o[kSymLines<T>][kSymRows];
+    if (act[0]) {
+#pragma unroll
+      for (int u = 0; u < kSymLines<T>; u++) {
+        const C<T> x0 = at(c[u], t);
+#pragma unroll
+        for (int i = 0; i < kSymRows; i++) {
+          e[u][i] = x0;
+          o[u][i] = mk<T>(T(0), T(0));
+        }
+      }
+      const C<T> *w = a.sym + (long)qb * kSymRows;
+      for (int r = 1; r <= H; r++, w += (long)nqb * kSymRows) {
+        C<T> cs[kSymRows];
+        ld_coef(w, cs);
+#pragma unroll
+        for (int u = 0; u < kSymLines<T>; u++) {
+          const C<T> s = at(c[u], t + P * r), d = at(c[u], t + P * (Q - r));
+#pragma unroll
+          for (int i = 0; i < kSymRows; i++) {
+            e[u][i].x += cs[i].x * s.x;
+            e[u][i].y += cs[i].x * s.y;
+            o[u][i].x += cs[i].y * d.x;
+            o[u][i].y += cs[i].y * d.y;
+          }
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kSymLines<T>; u++) {
+      if (!act[u]) continue;
+#pragma unroll
+      for (int i = 0; i < kSymRows; i++) {
+        const int q = qb * kSymRows + i;
+        if (q > H) break;
+        if (q == 0) {
+          st(c[u], t, e[u][i]);
+          continue;
+        }
+        const int p0 = t + P * q, p1 = t + P * (Q - q);
+        C<T> v0 = mk<T>(e[u][i].x + o[u][i].y, e[u][i].y - o[u][i].x);
+        C<T> v1 = mk<T>(e[u][i].x - o[u][i].y, e[u][i].y + o[u][i].x);
+        if (TW) {
+          v0 = cmul<T>(v0, __ldg(a.tw + p0));
+          v1 = cmul<T>(v1, __ldg(a.tw + p1));
+        }
+        st(c[u], p0, v0);
+        st(c[u], p1, v1);
+      }
+    }
+  }
+}
+
+// stage A: P butterflies of Q values; stage B: Q butterflies of P values.
+// at(line, position): the values' place in shared memory
+template <typename T, bool BIG, bool TW, typename Ld, typename At, typename St>
+__device__ __forceinline__ void stage_a(const Axis<T> &a, const Div &lines, Ld ld, At at, St st)
+{
+  if constexpr (BIG) {
+    if (a.sym) {
+      stage_sym<T, TW>(a, lines, ld, at, st);
+      return;
+    }
+  }
   stage<T, BIG, TW>(a.Q, a.P, 1, a.P, lines, a.tw, ld, st);
 }
 template <typename T, bool TW, typename Ld, typename St>
@@ -161,11 +288,11 @@ __global__ void __launch_bounds__(PlaneShape<T, BIG>::threads, 1)
   auto stx = [&](int y, int x, C<T> v) { xrow(y, x) = v; };
   if constexpr (!INV) {
     const C<T> *src = in + base;
-    stage_a<T, BIG, true>(ay, dx, [&](int x, int y) { return src[y * nx + x]; }, sty);
+    stage_a<T, BIG, true>(ay, dx, [&](int x, int y) { return src[y * nx + x]; }, ycol, sty);
     __syncthreads();
     stage_b<T, false>(ay, dx, ldy, sty);
     __syncthreads();
-    stage_a<T, BIG, true>(ax, dy, ldx, stx);
+    stage_a<T, BIG, true>(ax, dy, ldx, xrow, stx);
     __syncthreads();
     stage_b<T, false>(ax, dy, ldx, stx);
     __syncthreads();
@@ -185,14 +312,14 @@ __global__ void __launch_bounds__(PlaneShape<T, BIG>::threads, 1)
     __syncthreads();
     stage_b<T, true>(ax, dy, [&](int y, int x) { return exch<T>(xrow(y, x)); }, stx);
     __syncthreads();
-    stage_a<T, BIG, false>(ax, dy, ldx, stx);
+    stage_a<T, BIG, false>(ax, dy, ldx, xrow, stx);
     __syncthreads();
     stage_b<T, true>(ay, dx, ldy, sty);
     __syncthreads();
     const C<T> *ph = phi + base;
     const T *V = pot ? pot + base % ngrid : nullptr;
     C<T> *dst = out + base;
-    stage_a<T, BIG, false>(ay, dx, ldy, [&](int x, int y, C<T> v) {
+    stage_a<T, BIG, false>(ay, dx, ldy, ycol, [&](int x, int y, C<T> v) {
       const int o = y * nx + x;
       dst[o] = epilogue<T>(exch<T>(v), ph[o], V, o, ca, cb);
     });
@@ -221,9 +348,10 @@ __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>:
   const Div lines((unsigned)nl);
   const long es = ka.nxy;
   C<T> *d = data + blk * ngrid + c0;
+  auto at = [&](int c, int z) -> C<T> & { return S[z * L + c]; };
   auto lds = [&](int c, int z) { return S[z * L + c]; };
   auto sts = [&](int c, int z, C<T> v) { S[z * L + c] = v; };
-  stage_a<T, BIG, true>(az, lines, [&](int c, int z) { return d[z * es + c]; }, sts);
+  stage_a<T, BIG, true>(az, lines, [&](int c, int z) { return d[z * es + c]; }, at, sts);
   __syncthreads();
   with_radix<false>(az.P, [&](auto rc) {
     constexpr int RR = decltype(rc)::value;
@@ -259,7 +387,7 @@ __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>:
     }
   });
   __syncthreads();
-  stage_a<T, BIG, false>(az, lines, lds, [&](int c, int z, C<T> v) { d[z * es + c] = exch<T>(v); });
+  stage_a<T, BIG, false>(az, lines, lds, at, [&](int c, int z, C<T> v) { d[z * es + c] = exch<T>(v); });
 }
 
 // y lines of planes too large for shared memory: L consecutive x of one plane,
@@ -276,16 +404,17 @@ __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>:
   C<T> *d = data + pl * nx * ay.n + x0;
   auto ldg = [&](int c, int y) { return INV ? exch<T>(d[y * nx + c]) : d[y * nx + c]; };
   auto stg = [&](int c, int y, C<T> v) { d[y * nx + c] = INV ? exch<T>(v) : v; };
+  auto at = [&](int c, int y) -> C<T> & { return S[y * L + c]; };
   auto lds = [&](int c, int y) { return S[y * L + c]; };
   auto sts = [&](int c, int y, C<T> v) { S[y * L + c] = v; };
   if constexpr (!INV) {
-    stage_a<T, BIG, true>(ay, lines, ldg, sts);
+    stage_a<T, BIG, true>(ay, lines, ldg, at, sts);
     __syncthreads();
     stage_b<T, false>(ay, lines, lds, stg);
   } else {
     stage_b<T, true>(ay, lines, ldg, sts);
     __syncthreads();
-    stage_a<T, BIG, false>(ay, lines, lds, stg);
+    stage_a<T, BIG, false>(ay, lines, lds, at, stg);
   }
 }
 
@@ -308,11 +437,12 @@ __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>:
   for (unsigned i = threadIdx.x; i < count; i += blockDim.x) copy_async(S + i + dn(i) * (pitch - n), src + i);
   copy_wait();
   __syncthreads();
+  auto at = [&](int y, int x) -> C<T> & { return S[y * pitch + x]; };
   auto ldx = [&](int y, int x) { return S[y * pitch + x]; };
   auto stx = [&](int y, int x, C<T> v) { S[y * pitch + x] = v; };
   C<T> *dst = out + off;
   if constexpr (!INV) {
-    stage_a<T, BIG, true>(ax, lines, ldx, stx);
+    stage_a<T, BIG, true>(ax, lines, ldx, at, stx);
     __syncthreads();
     stage_b<T, false>(ax, lines, ldx, stx);
     __syncthreads();
@@ -321,7 +451,7 @@ __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>:
   } else {
     stage_b<T, true>(ax, lines, [&](int y, int x) { return exch<T>(S[y * pitch + x]); }, stx);
     __syncthreads();
-    stage_a<T, BIG, false>(ax, lines, ldx, stx);
+    stage_a<T, BIG, false>(ax, lines, ldx, at, stx);
     __syncthreads();
 #pragma unroll 4
     for (unsigned i = threadIdx.x; i < count; i += blockDim.x) {
@@ -343,9 +473,12 @@ namespace two {
 
 template <typename T> static Axis<T> axis_of(const AxisPlan &p)
 {
-  if constexpr (sizeof(T) == 4) return {p.n, p.P, p.Q, p.two32};
-  else return {p.n, p.P, p.Q, p.two64};
+  if constexpr (sizeof(T) == 4) return {p.n, p.P, p.Q, p.two32, p.sym32};
+  else return {p.n, p.P, p.Q, p.two64, p.sym64};
 }
+
+// threads that share one line in stage A: the butterflies, times the row blocks of stage_sym
+inline long line_threads(const AxisPlan &p) { return p.sym64 ? (long)p.P * ((p.Q / 2 + kSymRows) / kSymRows) : p.P; }
 
 template <typename K, typename... Args>
 static int launch(fbse_ctx *c, K kernel, long grid, int threads, size_t smem, Args... args)
@@ -357,10 +490,10 @@ static int launch(fbse_ctx *c, K kernel, long grid, int threads, size_t smem, Ar
   return FBSE_OK;
 }
 
-inline int round32(long v, int lo, int hi)
+inline int round32(long v, long lo, long hi)
 {
-  const long r = (v + 31) / 32 * 32;
-  return (int)(r < lo ? lo : r > hi ? hi : r);
+  const long r = (std::max(v, lo) + 31) / 32 * 32;
+  return (int)std::min(r, hi);
 }
 
 // threads of a plane CTA: the register file's share when as many CTAs as fit
@@ -368,14 +501,18 @@ inline int round32(long v, int lo, int hi)
 template <typename T, bool BIG> static int plane_threads(fbse_ctx *c, size_t smem, long grid)
 {
   const long fit = std::max<long>(1, std::min<long>((long)(228 * 1024 / (smem + 1024)), (grid + 151) / 152));
-  const long work = std::max(c->ax[0].P * c->ny, c->ax[1].P * c->nx);
-  return round32(std::min<long>(work, PlaneShape<T, BIG>::threads / fit), 128, PlaneShape<T, BIG>::threads);
+  const long px = line_threads(c->ax[0]), py = line_threads(c->ax[1]);
+  const long work = std::max(px * c->ny, py * c->nx);
+  return round32(std::min<long>(work, PlaneShape<T, BIG>::threads / fit / 32 * 32), std::max<long>(128, std::max(px, py)),
+                 PlaneShape<T, BIG>::threads);
 }
 
-// lines per tile: 256-byte segments, half of that when a launch would leave SMs idle
-template <typename T> static int tile_lines(long lines, long groups)
+// lines per tile of n points: 256-byte segments, half of that when a launch
+// would leave SMs idle, fewer when a long axis would take more than half an SM's
+// shared memory
+template <typename T> static int tile_lines(long lines, long groups, int n)
 {
-  const int full = 256 / (int)sizeof(C<T>);
+  const int full = std::max(2, std::min(256 / (int)sizeof(C<T>), (int)(112 * 1024 / ((n | 1) * sizeof(C<T>)))));
   int L = groups * ((lines + full - 1) / full) < 304 ? full / 2 : full;
   const long nt = (lines + L - 1) / L;
   return (int)((lines + nt - 1) / nt);  // even tiles
@@ -404,13 +541,13 @@ template <typename T> int two_z(fbse_ctx *c, C<T> *data, long nblk, const KinArg
 {
   using namespace two;
   const Axis<T> az = axis_of<T>(c->ax[2]);
-  const int L = tile_lines<T>(ka.nxy, nblk);
+  const int L = tile_lines<T>(ka.nxy, nblk, az.n);
   const int ntile = (int)((ka.nxy + L - 1) / L);
   const size_t smem = (size_t)az.n * L * sizeof(C<T>);
   if (az.Q > 16)
-    return launch(c, k_two_z<T, true>, nblk * ntile, round32((long)az.P * L, 64, LineShape<T, true>::threads), smem,
+    return launch(c, k_two_z<T, true>, nblk * ntile, round32(line_threads(c->ax[2]) * L, 64, LineShape<T, true>::threads), smem,
                   data, az, L, ntile, c->ngrid, ka);
-  return launch(c, k_two_z<T, false>, nblk * ntile, round32((long)az.P * L, 64, LineShape<T, false>::threads), smem,
+  return launch(c, k_two_z<T, false>, nblk * ntile, round32(line_threads(c->ax[2]) * L, 64, LineShape<T, false>::threads), smem,
                 data, az, L, ntile, c->ngrid, ka);
 }
 
@@ -418,11 +555,11 @@ template <typename T> int two_y(fbse_ctx *c, C<T> *data, long nblk, bool inv)
 {
   using namespace two;
   const Axis<T> ay = axis_of<T>(c->ax[1]);
-  const int L = tile_lines<T>(c->nx, nblk * c->nz);
+  const int L = tile_lines<T>(c->nx, nblk * c->nz, ay.n);
   const int ntile = (int)((c->nx + L - 1) / L);
   const size_t smem = (size_t)ay.n * L * sizeof(C<T>);
   const bool big = ay.Q > 16;
-  const int th = round32((long)ay.P * L, 64, big ? LineShape<T, true>::threads : LineShape<T, false>::threads);
+  const int th = round32(line_threads(c->ax[1]) * L, 64, big ? LineShape<T, true>::threads : LineShape<T, false>::threads);
   auto go = [&](auto k) { return launch(c, k, nblk * c->nz * ntile, th, smem, data, ay, (int)c->nx, L, ntile); };
   if (big) return inv ? go(k_two_y<T, true, true>) : go(k_two_y<T, true, false>);
   return inv ? go(k_two_y<T, false, true>) : go(k_two_y<T, false, false>);
@@ -434,11 +571,11 @@ int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T
   using namespace two;
   const Axis<T> ax = axis_of<T>(c->ax[0]);
   const long nlines = nblk * c->ny * c->nz;
-  const int L = tile_lines<T>(nlines, 1);
+  const int L = tile_lines<T>(nlines, 1, ax.n);
   const size_t smem = (size_t)(ax.n | 1) * L * sizeof(C<T>);
   const Div dn((unsigned)ax.n);
   const bool big = ax.Q > 16;
-  const int th = round32((long)ax.P * L, 64, big ? LineShape<T, true>::threads : LineShape<T, false>::threads);
+  const int th = round32(line_threads(c->ax[0]) * L, 64, big ? LineShape<T, true>::threads : LineShape<T, false>::threads);
   auto go = [&](auto k) {
     return launch(c, k, (nlines + L - 1) / L, th, smem, in, out, ax, dn, nlines, L, phi, pot, c->ngrid, ca, cb);
   };

@@ -705,6 +705,15 @@ static int ortho_diag_sigma_t(fbse_ctx *c, double *psitot, long n_, long *n_kept
     if (cudaMalloc(p, b) != cudaSuccess) { cudaGetLastError(); rc = set_err(c, FBSE_ERR_OOM, "ortho/diag scratch"); return false; }
     return true;
   };
+  // Ritz vectors of close pairs follow the rounding of the FP32 H psi: a change of
+  // 1e-7 in it moved vectors by up to 2e-3 (128 states, 86^3), so this step keeps
+  // one set of FFT kernels whatever H psi itself uses, and with it the vectors of
+  // earlier runs.  It applies H once per state, the filter thousands of times.
+  struct Steady {
+    fbse_ctx *c;
+    explicit Steady(fbse_ctx *c_) : c(c_) { c->steady = kMixed; }
+    ~Steady() { c->steady = 0; }
+  } steady(c);
   do {
     {
       void *a = nullptr, *b = nullptr;
