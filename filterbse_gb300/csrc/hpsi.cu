@@ -8,16 +8,20 @@
 // and scatters b_p(r) Y_m(r) sum_j' LS[j'][j] c[p][j'] into spin s of the
 // output (SO); the NL operator is the same with b^NL_p, a sign per channel and
 // no spin mixing.  Here one CTA per (atom, channel, group of states) gathers
-// the coefficients with one warp per (state, spin) (register accumulation,
-// warp reduction; the warps of a CTA share every table entry through L1) and
-// applies L.S (or the NL sign).  The scatter runs one thread per grid point
+// the coefficients with a few warps per state (register accumulation, one
+// reduction per warp, then over the warps in order) and applies L.S (or the NL
+// sign).  The scatter runs one thread per grid point
 // covered by any sphere (overlapping spheres of neighbouring atoms make it a
 // reduction, which the reference does with "omp atomic",
 // phamiltonian.c:295-303): each point's entries are summed in a fixed order,
 // so H psi is bit-identical from run to run.
-#include <cstdlib>
+#include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "fbse_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace fbse {
 
@@ -47,114 +51,180 @@ template <> ProjView<float> view<float>(fbse_ctx *c)
           p.nat * p.npts, p.nproj};
 }
 
-constexpr int kSW = 4;              // warps per CTA
-constexpr int kProjThreads = 32 * kSW;
 constexpr int kNC = 30;             // 5 radial channels x (2 spins x 3 m)
 
-// gather: one warp per (state, spin s'); each lane accumulates the 15
-// coefficients b_p conj(Y_m) psi_s' of its points, kGU points per iteration so
-// that the dependent loads (grid index, then psi) of several points are in
-// flight together; the grid indices of the next iteration are loaded before
-// the current iteration's arithmetic, so only the psi load is on the critical
-// path.  W warps per CTA (W / nspin states) share every table entry through
-// L1.  Then L.S (or the NL sign) per state:
-//   coef[((st*nat + a)*2 + ch)*30 + p*6 + j]
-template <typename T, int kGU, int MINB, int W>
-__global__ void __launch_bounds__(32 * W, MINB) k_proj_gather(const C<T> *__restrict__ psi, C<T> *__restrict__ coef,
-                                                              ProjView<T> pv, long nat, long nstates, long ngrid,
-                                                              int nspin, int ch0, double dv)
+// sum of v[i] over the 32 lanes, lane l left with the total of v[l]: 31
+// exchanges instead of 5 for each value
+template <typename T> __device__ __forceinline__ T transpose_sum(T (&v)[32], int lane)
 {
-  const long a = blockIdx.x;
+#pragma unroll
+  for (int h = 16; h >= 1; h >>= 1) {
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const T send = up ? v[i] : v[i + h];
+      const T keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+    }
+  }
+  return v[0];
+}
+
+// gather: the four warps of a CTA share the points of one (atom, channel, state),
+// both spins in one thread, so a table entry is loaded once for them.  Each lane
+// accumulates the 15 coefficients b_p conj(Y_m) psi_s' per spin of its points,
+// kGU points per iteration so that the dependent loads (grid index, then psi)
+// of several points are in flight together; the grid indices of the next
+// iteration are loaded before the current iteration's arithmetic, so only the
+// psi load is on the critical path.  The warps' sums meet in shared memory in
+// warp order, then L.S (or the NL sign) per state:
+//   coef[((st*nat + a)*2 + ch)*30 + p*6 + j]
+// CL: a few atoms leave SMs idle (FP64: and the few FP64 lanes of the busy ones are
+// what bounds the call), so a cluster of CTAs shares the points and the first one
+// adds the others' sums from their shared memory (gather_cluster).
+// Measured against a warp per (state, spin): mixed filter of 4 spinors at 96^3 with
+// 147 atoms 26.3 -> 20.8 ms (gather 58 us a call before, 12% of the warps), 920
+// single FP64 H psi of 15 atoms 589 -> 435 ms (119 us a call before, 30 CTAs); 16
+// spinors at 128^3 with 465 atoms 1248 -> 1222 us.
+// OWN: a warp per state with all its points, whose sums do not depend on a split
+// (the FP32 Rayleigh-Ritz step, fbse_ctx::steady).
+constexpr int kSW = 4;  // warps per CTA
+enum GatherMode { kShared, kCluster, kOwn };
+template <typename T, int kGU, int NSP, GatherMode MODE>
+__global__ void __launch_bounds__(32 * kSW)
+    k_proj_gather(const C<T> *__restrict__ psi, C<T> *__restrict__ coef, ProjView<T> pv, long nat, long ngrid, int ch0,
+                  double dv, int ncl, long nstates)
+{
+  constexpr bool CL = MODE == kCluster, OWN = MODE == kOwn;
+  const long a = CL ? blockIdx.x / ncl : blockIdx.x;
+  const int rank = CL ? (int)(blockIdx.x - a * ncl) : 0;
   const int ch = ch0 + blockIdx.y;  // 0: SO, 1: NL
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int spc = W / nspin;  // states per CTA
-  const long st = (long)blockIdx.z * spc + wid / nspin;
-  const int sp = wid % nspin;
-  const bool live = st < nstates;
-  const int np = pv.cnt[a];
-  const C<T> *ps = psi + (live ? st : 0) * nspin * ngrid + (long)sp * ngrid;
+  const long st = OWN ? (long)blockIdx.z * kSW + wid : blockIdx.z;
+  const int np = st < nstates ? pv.cnt[a] : 0;
+  const C<T> *ps = psi + st * NSP * ngrid;
   const T *rad = (ch == 0) ? pv.sop : pv.nlp;
   const int npj = pv.nproj;
   const long ebase = a * pv.npts;
-  T acc[30];
+  const int STEP = OWN ? 32 : 32 * kSW * (CL ? ncl : 1);  // points between a lane's points
+  T acc[NSP][32];
 #pragma unroll
-  for (int i = 0; i < 30; i++) acc[i] = T(0);
-  if (live) {
-    int jn[kGU];
+  for (int s = 0; s < NSP; s++)
+#pragma unroll
+    for (int i = 0; i < 32; i++) acc[s][i] = T(0);
+  const int first = OWN ? lane : (rank * kSW + wid) * 32 + lane;
+  int jn[kGU];
+#pragma unroll
+  for (int u = 0; u < kGU; u++) {
+    const int g = first + STEP * u;
+    jn[u] = g < np ? pv.jxyz[ebase + g] : -1;
+  }
+  for (int g0 = first; g0 < np; g0 += STEP * kGU) {
+    int jx[kGU];
+    C<T> v[kGU][NSP];
 #pragma unroll
     for (int u = 0; u < kGU; u++) {
-      const int g = lane + 32 * u;
+      jx[u] = jn[u];
+#pragma unroll
+      for (int s = 0; s < NSP; s++) v[u][s] = jx[u] >= 0 ? ps[s * ngrid + jx[u]] : mk<T>(T(0), T(0));
+    }
+#pragma unroll
+    for (int u = 0; u < kGU; u++) {
+      const int g = g0 + STEP * (kGU + u);
       jn[u] = g < np ? pv.jxyz[ebase + g] : -1;
     }
-    for (int g0 = lane; g0 < np; g0 += 32 * kGU) {
-      int jx[kGU];
-      C<T> v[kGU];
 #pragma unroll
-      for (int u = 0; u < kGU; u++) {
-        jx[u] = jn[u];
-        v[u] = jx[u] >= 0 ? ps[jx[u]] : mk<T>(T(0), T(0));
-      }
+    for (int u = 0; u < kGU; u++) {
+      if (jx[u] < 0) continue;
+      const long e = ebase + g0 + STEP * u;
+      T b[5];
 #pragma unroll
-      for (int u = 0; u < kGU; u++) {
-        const int g = g0 + 32 * (kGU + u);
-        jn[u] = g < np ? pv.jxyz[ebase + g] : -1;
-      }
+      for (int p = 0; p < 5; p++) b[p] = (p < npj) ? rad[p * pv.ne + e] : T(0);
 #pragma unroll
-      for (int u = 0; u < kGU; u++) {
-        if (jx[u] < 0) continue;
-        const long e = ebase + g0 + 32 * u;
-        T b[5];
+      for (int m = 0; m < 3; m++) {
+        const C<T> y = pv.y1[m * pv.ne + e];
 #pragma unroll
-        for (int p = 0; p < 5; p++) b[p] = (p < npj) ? rad[p * pv.ne + e] : T(0);
-#pragma unroll
-        for (int m = 0; m < 3; m++) {
-          const C<T> y = pv.y1[m * pv.ne + e];
+        for (int s = 0; s < NSP; s++) {
           // psi * conj(Y)
-          const T tr = v[u].x * y.x + v[u].y * y.y;
-          const T ti = v[u].y * y.x - v[u].x * y.y;
+          const T tr = v[u][s].x * y.x + v[u][s].y * y.y;
+          const T ti = v[u][s].y * y.x - v[u][s].x * y.y;
 #pragma unroll
           for (int p = 0; p < 5; p++) {
-            acc[2 * (p * 3 + m)] += b[p] * tr;
-            acc[2 * (p * 3 + m) + 1] += b[p] * ti;
+            acc[s][2 * (p * 3 + m)] += b[p] * tr;
+            acc[s][2 * (p * 3 + m) + 1] += b[p] * ti;
           }
         }
       }
     }
   }
+  __shared__ T part[kSW][NSP][32];
 #pragma unroll
-  for (int i = 0; i < 30; i++) {
-    T x = acc[i];
+  for (int s = 0; s < NSP; s++) part[wid][s][lane] = transpose_sum<T>(acc[s], lane);
+  __shared__ C<T> cf[OWN ? kSW * NSP : NSP][15];
+  auto sums = [&](int o, int n) {  // sum o of (spin, coefficient) over n CTAs of four warps
+    const int s = o / 15, i = o % 15;
+    T re = T(0), im = T(0);
+    for (int r = 0; r < n; r++) {
+      const T *pr = &part[0][s][2 * i];
+      if constexpr (CL) pr = cg::this_cluster().map_shared_rank(pr, r);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    acc[i] = x;
+      for (int q = 0; q < kSW; q++) {
+        re += pr[q * NSP * 32];
+        im += pr[q * NSP * 32 + 1];
+      }
+    }
+    cf[s][i] = mk<T>(re * (T)dv, im * (T)dv);
+  };
+  if constexpr (OWN) {
+    __syncthreads();
+    for (int o = threadIdx.x; o < kSW * NSP * 15; o += blockDim.x) {
+      const int row = o / 15, i = o % 15;
+      const T *pr = &part[row / NSP][row % NSP][2 * i];
+      cf[row][i] = mk<T>(pr[0] * (T)dv, pr[1] * (T)dv);
+    }
+    __syncthreads();
+  } else if constexpr (CL) {
+    cg::this_cluster().sync();
+    if (rank == 0 && threadIdx.x < NSP * 15) sums((int)threadIdx.x, ncl);
+    cg::this_cluster().sync();  // the first CTA has read the others' sums
+    if (rank != 0) return;
+  } else {
+    __syncthreads();
+    if (threadIdx.x < NSP * 15) sums((int)threadIdx.x, 1);
+    __syncthreads();
   }
-  __shared__ C<T> cf[W][15];
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < 15; i++) cf[wid][i] = mk<T>(acc[2 * i] * (T)dv, acc[2 * i + 1] * (T)dv);
-  }
-  __syncthreads();
-  for (int o = threadIdx.x; o < spc * kNC; o += blockDim.x) {
-    const int ls = o / kNC, q = o % kNC;
-    const long sg = (long)blockIdx.z * spc + ls;
-    if (sg >= nstates) continue;
-    const int p = q / 6, j = q % 6;
+  for (int o = threadIdx.x; o < (OWN ? kSW : 1) * kNC; o += blockDim.x) {
+    const int ls = o / kNC, q = o % kNC, p = q / 6, j = q % 6;
+    const long sg = OWN ? (long)blockIdx.z * kSW + ls : st;
+    if (OWN && sg >= nstates) continue;
+    const C<T>(*c)[15] = cf + ls * NSP;
     C<T> d = mk<T>(0, 0);
     if (ch == 0) {
       // d[p][j] = sum_j' LS[j'][j] c[p][j'], j' = 3 s' + m'   (phamiltonian.c:249-290)
-      for (int jp = 0; jp < 3 * nspin; jp++) {
+#pragma unroll
+      for (int jp = 0; jp < 3 * NSP; jp++) {
         const double2 l = pv.LS[jp * 6 + j];
-        const C<T> cc = cf[ls * nspin + jp / 3][p * 3 + jp % 3];
+        const C<T> cc = c[jp / 3][p * 3 + jp % 3];
         d.x += (T)l.x * cc.x - (T)l.y * cc.y;
         d.y += (T)l.x * cc.y + (T)l.y * cc.x;
       }
-    } else if (j / 3 < nspin) {
+    } else if (j / 3 < NSP) {
       // sign of the channel (phamiltonian.c:399-401), block diagonal in spin
       const T sgn = (p < npj) ? (T)pv.sgn[a * npj + p] : T(0);
-      d = cscale<T>(cf[ls * nspin + j / 3][p * 3 + j % 3], sgn);
+      d = cscale<T>(c[j / 3][p * 3 + j % 3], sgn);
     }
     coef[((sg * nat + a) * 2 + ch) * kNC + q] = d;
   }
+}
+
+// CTAs per (atom, channel, state) of the gather: a CTA on every SM for a single
+// state, from the system alone, so that a state's sums are the same in every batch
+static int gather_cluster(const fbse_ctx *c)
+{
+  const long pairs = std::max<long>(1, c->proj.nat * ((c->so ? 1 : 0) + (c->nl ? 1 : 0)));
+  int n = 1;
+  while (n < 8 && pairs * n < 152) n *= 2;
+  return n;
 }
 
 // point-major view of the table for the scatter (ProjDev::cov_j ...)
@@ -470,14 +540,44 @@ __global__ void __launch_bounds__(kScatterChunkPoints) k_proj_scatter_chunk(
   }
 }
 
-template <typename T, int kGU>
-static void launch_gather(fbse_ctx *c, dim3 g, const C<T> *in, C<T> *coef, const ProjView<T> &pv, long nstates, int ch0)
+template <typename T, int kGU, int NSP>
+static int launch_gather2(fbse_ctx *c, const C<T> *in, C<T> *coef, const ProjView<T> &pv, long nstates)
 {
-  // FP32 (mixed path): a register cap for 8 CTAs per SM (more warps in flight
-  // instead of more loads per warp); FP64: no cap (the cap spills there)
-  constexpr int kMinB = sizeof(T) == 4 ? 8 : 1;
-  k_proj_gather<T, kGU, kMinB, kSW><<<g, kProjThreads, 0, c->stream>>>(in, coef, pv, c->proj.nat, nstates, c->ngrid,
-                                                                      c->nspin, ch0, c->dv);
+  const int ncl = gather_cluster(c), ch0 = c->so ? 0 : 1, nch = (c->so ? 1 : 0) + (c->nl ? 1 : 0);
+  const dim3 g((unsigned)(c->proj.nat * ncl), (unsigned)nch, (unsigned)nstates);
+  if constexpr (sizeof(T) == 4) {
+    if (c->steady) {
+      const dim3 gs((unsigned)c->proj.nat, (unsigned)nch, (unsigned)((nstates + kSW - 1) / kSW));
+      k_proj_gather<T, kGU, NSP, kOwn><<<gs, 32 * kSW, 0, c->stream>>>(in, coef, pv, c->proj.nat, c->ngrid, ch0, c->dv, 1,
+                                                                      nstates);
+      return FBSE_OK;
+    }
+  }
+  if (ncl == 1) {
+    k_proj_gather<T, kGU, NSP, kShared><<<g, 32 * kSW, 0, c->stream>>>(in, coef, pv, c->proj.nat, c->ngrid, ch0, c->dv, 1,
+                                                                      nstates);
+    return FBSE_OK;
+  }
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)ncl;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = g;
+  cfg.blockDim = dim3(32 * kSW);
+  cfg.stream = c->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  FBSE_CUDA(c, cudaLaunchKernelEx(&cfg, k_proj_gather<T, kGU, NSP, kCluster>, in, coef, pv, c->proj.nat, c->ngrid, ch0,
+                                  c->dv, ncl, nstates));
+  return FBSE_OK;
+}
+
+template <typename T, int kGU>
+static int launch_gather(fbse_ctx *c, const C<T> *in, C<T> *coef, const ProjView<T> &pv, long nstates)
+{
+  return c->nspin == 2 ? launch_gather2<T, kGU, 2>(c, in, coef, pv, nstates)
+                       : launch_gather2<T, kGU, 1>(c, in, coef, pv, nstates);
 }
 
 template <typename T, bool SO, bool NL, int kG, int NPJ>
@@ -532,13 +632,8 @@ static int proj_gather(fbse_ctx *c, const C<T> *in, long nstates, long st0 = 0)
   int rc = ensure(c, &c->coef, &c->coef_bytes, need);
   if (rc) return rc;
   C<T> *coef = reinterpret_cast<C<T> *>(c->coef) + st0 * p.nat * 2 * kNC;
-  const long spc = kSW / c->nspin;
-  const long ggroups = (nstates + spc - 1) / spc;
-  if (ggroups > 65535 || p.nat > 2147483647L || nstates > 65535)
+  if (p.nat > 2147483647L / 8 || nstates > 65535)
     return set_err(c, FBSE_ERR_UNSUPPORTED, "projector grid too large");
-  const int ch0 = c->so ? 0 : 1;
-  const int nch = (c->so ? 1 : 0) + (c->nl ? 1 : 0);
-  dim3 gg((unsigned)p.nat, (unsigned)nch, (unsigned)ggroups);
   const ProjView<T> pv = view<T>(c);
   const std::string prob = std::string(sizeof(T) == 4 ? "fp32" : "fp64") + " states=" + std::to_string(nstates) +
                            " atoms=" + std::to_string(p.nat) + " points=" + std::to_string(p.ncov) +
@@ -547,10 +642,10 @@ static int proj_gather(fbse_ctx *c, const C<T> *in, long nstates, long st0 = 0)
   // choice); the gather writes only coef, so candidates run in place
   long gu = c->tune.gather_points;
   auto gather = [&](long v) -> int {
-    if (v == 1) launch_gather<T, 1>(c, gg, in, coef, pv, nstates, ch0);
-    else if (v == 4) launch_gather<T, 4>(c, gg, in, coef, pv, nstates, ch0);
-    else launch_gather<T, 2>(c, gg, in, coef, pv, nstates, ch0);
-    return launch_status(c);
+    const int r = v == 1 ? launch_gather<T, 1>(c, in, coef, pv, nstates)
+                : v == 4 ? launch_gather<T, 4>(c, in, coef, pv, nstates)
+                         : launch_gather<T, 2>(c, in, coef, pv, nstates);
+    return r ? r : launch_status(c);
   };
   if (gu == 0 && (rc = autotune(c, "projector gather points per lane", prob, {1, 2, 4}, gather, &gu))) return rc;
   if ((rc = gather(gu))) return rc;
