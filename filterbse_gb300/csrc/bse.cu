@@ -12,7 +12,8 @@
 //               per matrix element; here every pair density is formed and
 //               convolved in batches (the FFT engine's hartree mode), and each
 //               kernel becomes one complex GEMM over the grid,
-//               [pairs x N] x [N x pairs], with FP64 split-K partial sums.
+//               [pairs x N] x [N x pairs] on the tensor cores: exact slices for
+//               FP64 (exactgemm.cu), split TF32 on the mixed path (tcgemm.cu).
 //   solve       build_h0_mat / build_BSE_mat (bse_cplx/mod_bse.c:54-148) and
 //               bethe_salpeter (bse_cplx/bethe-salpeter.c:7-350):
 //               H = diag(e_a - e_i) - (K^d + K^x), Hermitian FP64 eigensolve on
@@ -198,6 +199,14 @@ static int cgemm_nt(fbse_ctx *c, const C<T> *A, int ma, const C<T> *B, int nb, l
     if (bse_tensor_cores(c))
       return tc_complex_nt<float>(c, reinterpret_cast<const float *>(A), ma, reinterpret_cast<const float *>(B), nb,
                                   L, false, scale, out);
+  } else {
+    // FP64: exact slices on the tensor cores; the SIMT kernel below where the
+    // product is short or their scratch does not fit
+    if (L >= kExactMin) {
+      const int rc = exact_nt(c, reinterpret_cast<const double *>(A), 2 * L, ma, reinterpret_cast<const double *>(B),
+                              2 * L, nb, L, kExactPlain, scale, out);
+      if (rc != FBSE_ERR_OOM) return rc;
+    }
   }
   long nchunk = std::max<long>(1, std::min<long>(64, L / 8192));
   // keep the partials bounded (64 x ma x nb complex doubles)
@@ -280,11 +289,17 @@ static int eh_kernels_t(fbse_ctx *c, const double *psi_qp, long nh, long ne, lon
   double2 *G = nullptr;
   const long maxrows = std::max(ne * ne, std::max(nh * nh, nx));
   auto fail = [&](const char *m) { cudaGetLastError(); rc = set_err(c, FBSE_ERR_OOM, m); };
-  if (cudaMalloc(&P, (size_t)maxrows * N * sizeof(C<T>)) != cudaSuccess) fail("bse pair densities");
-  else if (cudaMalloc(&Q, (size_t)maxrows * N * sizeof(C<T>)) != cudaSuccess) fail("bse pair densities");
-  else if (cudaMalloc(&wk, (size_t)2 * batch * N * sizeof(C<T>)) != cudaSuccess) fail("bse fft scratch");
-  else if (cudaMalloc(&dpairs, (size_t)maxrows * sizeof(int2)) != cudaSuccess) fail("bse pairs");
-  else if (cudaMalloc(&G, (size_t)(ne * ne) * (nh * nh) * sizeof(double2)) != cudaSuccess) fail("bse G");
+  auto get = [&](auto **p, size_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    release(c, kSlotTc);  // an earlier product's scratch
+    return cudaMalloc(p, bytes) == cudaSuccess;
+  };
+  if (!get(&P, (size_t)maxrows * N * sizeof(C<T>))) fail("bse pair densities");
+  else if (!get(&Q, (size_t)maxrows * N * sizeof(C<T>))) fail("bse pair densities");
+  else if (!get(&wk, (size_t)2 * batch * N * sizeof(C<T>))) fail("bse fft scratch");
+  else if (!get(&dpairs, (size_t)maxrows * sizeof(int2))) fail("bse pairs");
+  else if (!get(&G, (size_t)(ne * ne) * (nh * nh) * sizeof(double2))) fail("bse G");
   std::vector<int2> pr;
   do {
     if (rc) break;

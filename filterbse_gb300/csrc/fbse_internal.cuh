@@ -205,6 +205,15 @@ inline int cached(fbse_ctx *c, int slot, size_t need, void **out)
   *out = c->cache[slot];
   return rc;
 }
+// gives a kept buffer back (after the stream's work that uses it)
+inline void release(fbse_ctx *c, int slot)
+{
+  if (!c->cache[slot]) return;
+  cudaStreamSynchronize(c->stream);
+  cudaFree(c->cache[slot]);
+  c->cache[slot] = nullptr;
+  c->cache_bytes[slot] = 0;
+}
 // reads (and clears) the device error flags of the kernels with bounded waits
 int check_dev_status(fbse_ctx *c);
 
@@ -301,6 +310,16 @@ int zpass_kinetic(fbse_ctx *c, float2 *data, long nblk);
 template <typename S>
 int tc_complex_nt(fbse_ctx *c, const S *A, int ma, const S *B, int nb, long L, bool conj_a, double scale,
                   double2 *out);
+
+// FP64 products on the tensor cores by exact integer slices (exactgemm.cu):
+//   out[i][j] = scale * sum_l f(A_i[l]) B_j[l] over L values of each row; rows are
+//   lda / ldb doubles apart and hold real values, or complex ones as (re, im)
+// Scratch is kept in the context; FBSE_ERR_OOM leaves nothing enqueued.
+enum ExactKind { kExactReal, kExactPlain, kExactConj };  // real; complex; complex with f = conj
+// a product shorter than this is not worth the slicing
+constexpr long kExactMin = 2048;
+int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, long ldb, int nb, long L, ExactKind kind,
+             double scale, double2 *out);
 
 // reductions / vector ops (filter.cu) ------------------------------------------
 template <typename T>

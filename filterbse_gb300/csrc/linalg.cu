@@ -644,6 +644,13 @@ template <typename T>
 static int gram_t(fbse_ctx *c, const double *A, const double *B, int n, long L, double2 *out, double scale,
                   double2 *part, int nchunk, long kchunk)
 {
+  if constexpr (sizeof(T) == 8) {
+    if (L >= kExactMin) {
+      const long ld = (c->is_complex + 1) * L;
+      const int rc = exact_nt(c, A, ld, n, B, ld, n, L, c->is_complex ? kExactConj : kExactReal, scale, out);
+      if (rc != FBSE_ERR_OOM) return rc;
+    }
+  }
   const int nt = (n + 63) / 64;
   dim3 g(nt * (nt + 1) / 2, 1, nchunk);
   // resident CTAs per SM: one (no register cap) or two (a cap of 128
@@ -702,8 +709,13 @@ static int ortho_diag_sigma_t(fbse_ctx *c, double *psitot, long n_, long *n_kept
   const long kchunk = (L + nchunk - 1) / nchunk;
   const int nrb = (int)((L + 127) / 128);
   auto alloc = [&](void **p, size_t b) -> bool {
-    if (cudaMalloc(p, b) != cudaSuccess) { cudaGetLastError(); rc = set_err(c, FBSE_ERR_OOM, "ortho/diag scratch"); return false; }
-    return true;
+    if (cudaMalloc(p, b) == cudaSuccess) return true;
+    cudaGetLastError();
+    release(c, kSlotTc);  // an earlier product's scratch
+    if (cudaMalloc(p, b) == cudaSuccess) return true;
+    cudaGetLastError();
+    rc = set_err(c, FBSE_ERR_OOM, "ortho/diag scratch");
+    return false;
   };
   // Ritz vectors of close pairs follow the rounding of the FP32 H psi: a change of
   // 1e-7 in it moved vectors by up to 2e-3 (128 states, 86^3), so this step keeps
@@ -962,6 +974,17 @@ int gram_slab(fbse_ctx *c, const double *A, long na, const double *B, long nb, l
   const long stride = (long)(c->is_complex + 1) * L;
   if (na < 1 || nb < 1 || off < 0 || len < 1 || off + len > L || na > 65535 * 64L || nb > 65535 * 64L)
     return set_err(c, FBSE_ERR_ARG, "fbse_gram: sizes");
+  if (len >= kExactMin && na <= 65535 && nb <= 65535) {
+    const int w = c->is_complex + 1;
+    void *o = nullptr;
+    int rx = cached(c, kSlotProj, (size_t)na * nb * sizeof(double2), &o);
+    if (!rx)
+      rx = exact_nt(c, A + off * w, stride, (int)na, B + off * w, stride, (int)nb, len,
+                    c->is_complex ? kExactConj : kExactReal, c->dv, static_cast<double2 *>(o));
+    if (!rx && d2h(c->stream, out_host, o, (size_t)na * nb * sizeof(double2)) != cudaSuccess)
+      rx = set_err(c, FBSE_ERR_CUDA, "fbse_gram: download");
+    if (rx != FBSE_ERR_OOM) return rx;
+  }
   const int nchunk = (int)std::min<long>(std::max<long>(1, len / 8192), 256);
   const long kchunk = (len + nchunk - 1) / nchunk;
   double2 *part = nullptr, *sum = nullptr;
