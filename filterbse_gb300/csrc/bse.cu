@@ -31,7 +31,7 @@
 
 namespace fbse {
 
-int jacobi_eig_dev(fbse_ctx *c, double2 *A, double2 *V, int n, std::vector<double> &w);
+int jacobi_eig_dev(fbse_ctx *c, double2 *A, double2 *V, int n, std::vector<double> &w, bool real);
 int zgemm_dev(fbse_ctx *c, int m, int p, int k, const double2 *A, int lda, bool ah, const double2 *B, int ldb, bool bh,
               double2 *C, int ldc);
 int forward_fft64(fbse_ctx *c, double2 *data, double2 *work);
@@ -769,7 +769,7 @@ int fbse_bse_solve(fbse_ctx *c, const double *eval_qp_host, long n_qp, long n_h,
       break;
     }
     std::vector<double> w;
-    if ((rc = jacobi_eig_dev(c, T1, V, (int)n, w))) break;
+    if ((rc = jacobi_eig_dev(c, T1, V, (int)n, w, false))) break;
     std::vector<int> perm(n);
     for (long i = 0; i < n; i++) perm[i] = (int)i;
     std::sort(perm.begin(), perm.end(), [&](int a, int b) { return w[a] < w[b]; });

@@ -154,8 +154,9 @@ struct fbse_ctx {
   double *red = nullptr; size_t red_bytes = 0;   // reduction partials
   int *dstatus = nullptr;                        // device error flags of kernels with bounded waits
   int tc_poisoned = 0;  // a tensor-core wait timed out: MMAs may still be in flight, the path is refused
-  // the FP32 Rayleigh-Ritz step (ortho_diag_sigma) is running: H psi takes the
-  // mixed-radix FFT kernels on every axis that the register-resident ones do not
+  // the Rayleigh-Ritz step (ortho_diag_sigma) is running: H psi takes the mixed-radix
+  // FFT kernels on every axis that the register-resident ones do not, and the
+  // gather a warp per state
   int steady = 0;
   int nsm = 0;          // multiprocessors of the device (queried on first use)
   // large buffers kept between calls (grown on demand, freed by fbse_destroy):

@@ -87,7 +87,7 @@ template <typename T> __device__ __forceinline__ T transpose_sum(T (&v)[32], int
 // single FP64 H psi of 15 atoms 589 -> 435 ms (119 us a call before, 30 CTAs); 16
 // spinors at 128^3 with 465 atoms 1248 -> 1222 us.
 // OWN: a warp per state with all its points, whose sums do not depend on a split
-// (the FP32 Rayleigh-Ritz step, fbse_ctx::steady).
+// (the Rayleigh-Ritz step, fbse_ctx::steady).
 constexpr int kSW = 4;  // warps per CTA
 enum GatherMode { kShared, kCluster, kOwn };
 template <typename T, int kGU, int NSP, GatherMode MODE>
@@ -545,13 +545,11 @@ static int launch_gather2(fbse_ctx *c, const C<T> *in, C<T> *coef, const ProjVie
 {
   const int ncl = gather_cluster(c), ch0 = c->so ? 0 : 1, nch = (c->so ? 1 : 0) + (c->nl ? 1 : 0);
   const dim3 g((unsigned)(c->proj.nat * ncl), (unsigned)nch, (unsigned)nstates);
-  if constexpr (sizeof(T) == 4) {
-    if (c->steady) {
-      const dim3 gs((unsigned)c->proj.nat, (unsigned)nch, (unsigned)((nstates + kSW - 1) / kSW));
-      k_proj_gather<T, kGU, NSP, kOwn><<<gs, 32 * kSW, 0, c->stream>>>(in, coef, pv, c->proj.nat, c->ngrid, ch0, c->dv, 1,
-                                                                      nstates);
-      return FBSE_OK;
-    }
+  if (c->steady) {
+    const dim3 gs((unsigned)c->proj.nat, (unsigned)nch, (unsigned)((nstates + kSW - 1) / kSW));
+    k_proj_gather<T, kGU, NSP, kOwn><<<gs, 32 * kSW, 0, c->stream>>>(in, coef, pv, c->proj.nat, c->ngrid, ch0, c->dv, 1,
+                                                                    nstates);
+    return FBSE_OK;
   }
   if (ncl == 1) {
     k_proj_gather<T, kGU, NSP, kShared><<<g, 32 * kSW, 0, c->stream>>>(in, coef, pv, c->proj.nat, c->ngrid, ch0, c->dv, 1,

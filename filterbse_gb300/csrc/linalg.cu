@@ -16,8 +16,6 @@
 //   7. sigma_i = ||r_i|| / ||Psi_f,i||, states normalised (normalize_all).
 // H is applied n times in total instead of the reference's 3n, and the Ritz
 // vectors' residuals come from the same two GEMMs that build the vectors.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <cmath>
 #include <numeric>
@@ -28,8 +26,6 @@
 
 #include "fbse_internal.cuh"
 
-namespace cg = cooperative_groups;
-
 namespace fbse {
 
 int pack_states(fbse_ctx *c, const double *src, void *dst, long nsrc);
@@ -38,7 +34,7 @@ int unpack_states(fbse_ctx *c, const void *src, double *dst, long ndst);
 // ---------------------------------------------------------------------------
 // C[i][j] (+)= sum_l conj(A[i][l]) B[j][l]  over a K-chunk, i < n, j < n.
 // A, B: n vectors of length L (complex: interleaved FP64 pairs; real: FP64).
-// Tile 64 x 64 outputs per CTA, 256 threads x (4 x 4) outputs, K step 16.
+// Tile 64 x 64 outputs per CTA (32 x 32 in FP64), 256 threads, K step 16.
 // Compute type T (float for the mixed path, double for the FP64 path);
 // partials are written in FP64: part[chunk][i][j].  Both products this file
 // forms (Psi^H Psi and Psi^H H Psi) are Hermitian, so only tiles with
@@ -59,36 +55,40 @@ template <typename T> __device__ __forceinline__ void two_sum_acc(T &hi, T &lo, 
   lo += err;
 }
 
-template <typename T, bool CPLX, int MINB>
+template <typename T, bool CPLX, int MINB, int TM = 64>
 __global__ void __launch_bounds__(256, MINB) k_gram(const double *__restrict__ A, const double *__restrict__ B, int n,
                                               long L, long kchunk, double2 *__restrict__ part)
 {
-  constexpr int TM = 64, TK = 16;
+  constexpr int TK = 16, R = TM / 16;
   using E = typename std::conditional<CPLX, C<T>, T>::type;
   __shared__ E As[TK][TM + 1];
   __shared__ E Bs[TK][TM + 1];
-  // tile pair (ti, tj), ti <= tj, from the linear index
-  const int nt = (n + TM - 1) / TM;
-  int ti = 0, rem = blockIdx.x;
+  // pair (ti, tj), ti <= tj, of 64 x 64 blocks from the linear index, and the tile's
+  // corner in it.  Both halves of a diagonal block are formed (they differ in their
+  // last bits), so the tile size changes no value
+  constexpr int S = 64 / TM;
+  const int nt = (n + 63) / 64;
+  int ti = 0, rem = blockIdx.x / (S * S);
   while (rem >= nt - ti) { rem -= nt - ti; ti++; }
-  const int tj = ti + rem;
-  const int i0 = ti * TM, j0 = tj * TM;
+  const int tj = ti + rem, sub = blockIdx.x % (S * S);
+  const int i0 = ti * 64 + sub / S * TM, j0 = tj * 64 + sub % S * TM;
+  if (i0 >= n || j0 >= n) return;
   const long k0 = blockIdx.z * kchunk;
   const long k1 = min(L, k0 + kchunk);
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
   // FP32: the sums of each K step of 16 products are added into a
   // float-float pair (hi, lo) with TwoSum (Knuth), so the long sums over the
   // grid keep about 48 bits; FP64: plain accumulation
-  T accr[4][4], acci[4][4];
-  T hir[4][4], hii[4][4], lor[4][4], loi[4][4];
+  T accr[R][R], acci[R][R];
+  T hir[R][R], hii[R][R], lor[R][R], loi[R][R];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < R; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) { accr[a][b] = 0; acci[a][b] = 0; hir[a][b] = hii[a][b] = lor[a][b] = loi[a][b] = 0; }
+    for (int b = 0; b < R; b++) { accr[a][b] = 0; acci[a][b] = 0; hir[a][b] = hii[a][b] = lor[a][b] = loi[a][b] = 0; }
   for (long kb = k0; kb < k1; kb += TK) {
-    // load: 64 rows x 16 k for A and B; thread t loads rows (t / 16) + 16 q, k = t % 16
+    // load: TM rows x 16 k for A and B; thread t loads rows (t / 16) + 16 q, k = t % 16
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < R; q++) {
       const int r = ty + 16 * q, kk = tx;
       const long k = kb + kk;
       const bool okA = (i0 + r < n) && (k < k1);
@@ -106,9 +106,9 @@ __global__ void __launch_bounds__(256, MINB) k_gram(const double *__restrict__ A
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < TK; kk++) {
-      T ar[4], ai[4], br[4], bi[4];
+      T ar[R], ai[R], br[R], bi[R];
 #pragma unroll
-      for (int a = 0; a < 4; a++) {
+      for (int a = 0; a < R; a++) {
         if constexpr (CPLX) {
           const C<T> u = As[kk][ty + 16 * a], v = Bs[kk][tx + 16 * a];
           ar[a] = u.x; ai[a] = u.y; br[a] = v.x; bi[a] = v.y;
@@ -118,19 +118,28 @@ __global__ void __launch_bounds__(256, MINB) k_gram(const double *__restrict__ A
         }
       }
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+      for (int a = 0; a < R; a++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-          // conj(a) * b
-          accr[a][b] += ar[a] * br[b] + (CPLX ? ai[a] * bi[b] : T(0));
-          if (CPLX) acci[a][b] += ar[a] * bi[b] - ai[a] * br[b];
+        for (int b = 0; b < R; b++) {
+          // conj(a) * b; FP64 spells its roundings out (they decide phases, see the caller)
+          if constexpr (sizeof(T) == 8) {
+            if constexpr (CPLX) {
+              accr[a][b] = __dadd_rn(accr[a][b], __fma_rn(ar[a], br[b], __dmul_rn(ai[a], bi[b])));
+              acci[a][b] = __dadd_rn(acci[a][b], __fma_rn(ar[a], bi[b], -__dmul_rn(ai[a], br[b])));
+            } else {
+              accr[a][b] = __dadd_rn(accr[a][b], __dmul_rn(ar[a], br[b]));
+            }
+          } else {
+            accr[a][b] += ar[a] * br[b] + (CPLX ? ai[a] * bi[b] : T(0));
+            if (CPLX) acci[a][b] += ar[a] * bi[b] - ai[a] * br[b];
+          }
         }
     }
     if constexpr (sizeof(T) == 4) {
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+      for (int a = 0; a < R; a++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
+        for (int b = 0; b < R; b++) {
           two_sum_acc(hir[a][b], lor[a][b], accr[a][b]);
           accr[a][b] = 0;
           if (CPLX) {
@@ -143,9 +152,9 @@ __global__ void __launch_bounds__(256, MINB) k_gram(const double *__restrict__ A
   }
   double2 *P = part + (long)blockIdx.z * n * n;
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < R; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
+    for (int b = 0; b < R; b++) {
       const int i = i0 + ty + 16 * a, j = j0 + tx + 16 * b;
       double vr = (double)accr[a][b], vi = (double)acci[a][b];
       if constexpr (sizeof(T) == 4) {
@@ -202,10 +211,30 @@ int zgemm_dev(fbse_ctx *c, int m, int p, int k, const double2 *A, int lda, bool 
 // ---------------------------------------------------------------------------
 // Hermitian eigensolver: cyclic two-sided Jacobi with the round-robin pairing
 // (n/2 disjoint rotations per round, n-1 rounds per sweep), one cooperative
-// launch per sweep with two grid-wide barriers per round (rotation
-// parameters, then the two-sided update of A and V).
-// A (n x n, row-major, Hermitian) is diagonalised in place; V accumulates the
-// unitary so that A_in = V diag(A_out) V^H.
+// launch per sweep.  A (n x n, row-major, Hermitian) is diagonalised; V
+// accumulates the unitary so that A_in = V diag(A_out) V^H.
+//
+// The pairs of a round cover every index once, so every element of A lies in one
+// 2 x 2 block (row pair a, column pair b) and every element of V in one 1 x 2
+// block (row i, column pair b).  A block is rotated from both sides at once,
+// A_blk <- U_a^H A_blk U_b:
+//   rows:    new p = cs a_p - sn e^{i phi} a_q,   new q = sn a_p + cs e^{i phi} a_q
+//   columns: new p = cs a_p - sn e^{-i phi} a_q,  new q = sn a_p + cs e^{-i phi} a_q
+// and the rotated pair's off-diagonal element, zero in exact arithmetic, is set to
+// zero.  A dummy index (q = n for odd n) carries the identity.
+//
+// The arithmetic of every element and rotation is fixed: eigenvectors of a
+// rank-deficient overlap carry phases that follow the last bits of this sum order
+// (a filtered set's null directions are rounding noise, and every rotation passes
+// a phase on), so a different but equally accurate formula turns whole Ritz sets.
+//
+// A round is a chain of latencies (the pair's elements from L2, the rotation's
+// roots, the update, the grid barrier), so it has one barrier: a round reads A from
+// one buffer and writes every element to another, and each tile of 8 x 8 blocks (or
+// 8 pairs x 32 rows of V) computes the rotations of its own 16 pairs.  Tiles of 64
+// threads spread the FP64 work (2 lanes per clock and SM) over every SM from n = 128
+// on.  Measured per round against two barriers and a thread per block of the whole
+// matrix: n = 128 12.5 -> 6.6 us, n = 196 12.7 -> 6.9 us, n = 115 real 12.4 -> 6.6 us.
 // ---------------------------------------------------------------------------
 struct Rot {
   double cs, sn, pr, pi;  // U = D J:  U_pp = cs, U_pq = sn, U_qp = -sn e^{-i phi}, U_qq = cs e^{-i phi}
@@ -221,122 +250,187 @@ __device__ __forceinline__ void rr_pair(int r, int slot, int m, int &p, int &q)
   q = max(a, b);
 }
 
-__global__ void k_jacobi_sweep(double2 *__restrict__ A, double2 *__restrict__ V, int n, int m, Rot *__restrict__ rot,
-                               double *__restrict__ off)
+// the rotation that zeroes the pair's off-diagonal element
+__device__ __forceinline__ Rot pair_rotation(const double2 *__restrict__ A, int n, int p, int q)
 {
-  cg::grid_group grid = cg::this_grid();
-  const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const long nth = (long)gridDim.x * blockDim.x;
-  const int half = m / 2;
-  const long nblk = (long)half * half;  // 2 x 2 blocks of A, one per (row pair, column pair)
+  Rot R{1.0, 0.0, 1.0, 0.0, p, q};
+  if (q < n) {
+    const double app = __ldcg(&A[(long)p * n + p]).x, aqq = __ldcg(&A[(long)q * n + q]).x;
+    const double2 apq = __ldcg(&A[(long)p * n + q]);
+    const double mag = hypot(apq.x, apq.y);
+    if (mag > 1e-300 && mag > 1e-18 * sqrt(fabs(app * aqq))) {
+      const double tau = (aqq - app) / (2.0 * mag);
+      const double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+      R.cs = 1.0 / sqrt(1.0 + t * t);
+      R.sn = t * R.cs;
+      R.pr = apq.x / mag;  // e^{i phi}
+      R.pi = apq.y / mag;
+    }
+  }
+  return R;
+}
+
+// grid-wide barrier number `gen` (1, 2, ..) of a cooperative launch; bounded
+__device__ __forceinline__ bool grid_barrier(unsigned *counter, unsigned target)
+{
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+    int done = 0;
+    for (long i = 0; i < (1L << 26) && !done; i++) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+      done = (int)(v - target) >= 0;
+    }
+    ok = done;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+constexpr int kJT = 8, kJRows = 32, kJThreads = 64;  // pairs per tile side, V rows per tile
+
+// REAL: every imaginary part is zero and stays zero.  off[0..1]: off-diagonal and
+// diagonal sums of squares, off[2]: nonzero when a barrier gave up, then the CTAs'
+// partial sums.  count0: barriers of earlier launches on this counter.
+template <bool REAL>
+__global__ void __launch_bounds__(kJThreads) k_jacobi_sweep(double2 *__restrict__ A0, double2 *__restrict__ A1,
+                                                            double2 *__restrict__ V, int n, int m,
+                                                            unsigned *__restrict__ counter, unsigned count0,
+                                                            double *__restrict__ off)
+{
+  const int half = m / 2, T = (half + kJT - 1) / kJT, TV = (n + kJRows - 1) / kJRows;
+  const int na = T * T, ntile = na + T * TV;
+  const int tid = threadIdx.x;
+  __shared__ Rot rot[2 * kJT];
+  // (p, q) <- (cs p - sn w q, sn p + cs w q), w the (conjugated) phase; the roundings
+  // are spelled out (row: of which product of w q's imaginary part)
+  auto turn = [](const Rot &R, double2 w, double2 &ap, double2 &aq, bool row) {
+    double2 x;
+    x.x = REAL ? __dmul_rn(w.x, aq.x) : __fma_rn(w.x, aq.x, -__dmul_rn(w.y, aq.y));
+    x.y = row ? __fma_rn(w.y, aq.x, __dmul_rn(w.x, aq.y)) : __fma_rn(w.x, aq.y, __dmul_rn(w.y, aq.x));
+    const double2 y = ap;
+    ap.x = __fma_rn(R.cs, y.x, -__dmul_rn(R.sn, x.x));
+    aq.x = __fma_rn(R.sn, y.x, __dmul_rn(R.cs, x.x));
+    if (REAL) return;
+    ap.y = __fma_rn(R.cs, y.y, -__dmul_rn(R.sn, x.y));
+    aq.y = __fma_rn(R.sn, y.y, __dmul_rn(R.cs, x.y));
+  };
+  unsigned gen = count0;
   for (int r = 0; r < m - 1; r++) {
-    // phase 1: rotation parameters for the n/2 pairs of this round
-    for (long s = tid; s < half; s += nth) {
-      int p, q;
-      rr_pair(r, (int)s, m, p, q);
-      Rot R{1.0, 0.0, 1.0, 0.0, p, q};
-      if (q < n) {
-        const double app = A[(long)p * n + p].x, aqq = A[(long)q * n + q].x;
-        const double2 apq = A[(long)p * n + q];
-        const double mag = hypot(apq.x, apq.y);
-        if (mag > 1e-300 && mag > 1e-18 * sqrt(fabs(app * aqq))) {
-          const double tau = (aqq - app) / (2.0 * mag);
-          const double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-          R.cs = 1.0 / sqrt(1.0 + t * t);
-          R.sn = t * R.cs;
-          R.pr = apq.x / mag;  // e^{i phi}
-          R.pi = apq.y / mag;
+    const double2 *src = (r & 1) ? A1 : A0;
+    double2 *dst = (r & 1) ? A0 : A1;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+      const bool on_a = tile < na;
+      // tiles of pairs; V: pairs tb, rows ta
+      const int ta = on_a ? tile / T : (tile - na) % TV, tb = on_a ? tile % T : (tile - na) / TV;
+      // this thread's block(s) on their way while the rotations are formed
+      const int la = tid / kJT, lb = tid % kJT, sa = ta * kJT + la, sb = tb * kJT + lb;
+      int pa = 0, qa = n, pb = 0, qb = n;
+      const bool live = sb < half && (!on_a || sa < half);
+      if (live) {
+        rr_pair(r, sb, m, pb, qb);
+        if (on_a) rr_pair(r, sa, m, pa, qa);
+      }
+      double2 x[2][2];
+      double2 v[kJRows / kJT][2];
+      if (live && on_a) {
+        x[0][0] = __ldcg(&src[(long)pa * n + pb]);
+        x[0][1] = qb < n ? __ldcg(&src[(long)pa * n + qb]) : make_double2(0, 0);
+        x[1][0] = qa < n ? __ldcg(&src[(long)qa * n + pb]) : make_double2(0, 0);
+        x[1][1] = qa < n && qb < n ? __ldcg(&src[(long)qa * n + qb]) : make_double2(0, 0);
+      } else if (live && qb < n) {
+#pragma unroll
+        for (int u = 0; u < kJRows / kJT; u++) {
+          const int row = ta * kJRows + la + kJT * u;
+          if (row >= n) continue;
+          v[u][0] = __ldcg(&V[(long)row * n + pb]);
+          v[u][1] = __ldcg(&V[(long)row * n + qb]);
         }
       }
-      rot[s] = R;
-    }
-    grid.sync();
-    // phase 2: the pairs of a round cover every index once, so every element
-    // of A lies in one 2 x 2 block (row pair a, column pair b) and every
-    // element of V in one 1 x 2 block (row i, column pair b).  A block is
-    // rotated from both sides at once, A_blk <- U_a^H A_blk U_b:
-    //   rows:    new p = cs a_p - sn e^{i phi} a_q,   new q = sn a_p + cs e^{i phi} a_q
-    //   columns: new p = cs a_p - sn e^{-i phi} a_q,  new q = sn a_p + cs e^{-i phi} a_q
-    // and the rotated pair's off-diagonal element, zero in exact arithmetic,
-    // is set to zero.  A dummy index (q = n for odd n) carries the identity.
-    for (long w = tid; w < nblk + (long)n * half; w += nth) {
-      if (w < nblk) {
-        const Rot Ra = rot[w / half], Rb = rot[w % half];
-        const bool qa = Ra.q < n, qb = Rb.q < n;
-        double2 x[2][2];
-        x[0][0] = A[(long)Ra.p * n + Rb.p];
-        x[0][1] = qb ? A[(long)Ra.p * n + Rb.q] : make_double2(0, 0);
-        x[1][0] = qa ? A[(long)Ra.q * n + Rb.p] : make_double2(0, 0);
-        x[1][1] = qa && qb ? A[(long)Ra.q * n + Rb.q] : make_double2(0, 0);
-        const double2 ea = make_double2(Ra.pr, Ra.pi);
+      __syncthreads();  // the previous tile is done with rot
+      if (tid < 2 * kJT) {
+        const int s = (tid < kJT ? ta * kJT : tb * kJT - kJT) + tid;
+        if (s < half && (on_a || tid >= kJT)) {
+          int p, q;
+          rr_pair(r, s, m, p, q);
+          rot[tid] = pair_rotation(src, n, p, q);
+        }
+      }
+      __syncthreads();
+      if (!live) continue;
+      const Rot &Rb = rot[kJT + lb];
+      const double2 wb = make_double2(Rb.pr, -Rb.pi);
+      if (on_a) {
+        const Rot &Ra = rot[la];
+        const double2 wa = make_double2(Ra.pr, Ra.pi);
+        turn(Ra, wa, x[0][0], x[1][0], true);
+        turn(Ra, wa, x[0][1], x[1][1], true);
+        turn(Rb, wb, x[0][0], x[0][1], false);
+        turn(Rb, wb, x[1][0], x[1][1], false);
+        if (sa == sb && !(Ra.cs == 1.0 && Ra.sn == 0.0)) x[0][1] = x[1][0] = make_double2(0, 0);
+        __stcg(&dst[(long)pa * n + pb], x[0][0]);
+        if (qb < n) __stcg(&dst[(long)pa * n + qb], x[0][1]);
+        if (qa < n) __stcg(&dst[(long)qa * n + pb], x[1][0]);
+        if (qa < n && qb < n) __stcg(&dst[(long)qa * n + qb], x[1][1]);
+      } else if (qb < n) {
 #pragma unroll
-        for (int c = 0; c < 2; c++) {
-          const double2 ap = x[0][c], aq = x[1][c];
-          const double2 eaq = make_double2(ea.x * aq.x - ea.y * aq.y, ea.x * aq.y + ea.y * aq.x);
-          x[0][c] = make_double2(Ra.cs * ap.x - Ra.sn * eaq.x, Ra.cs * ap.y - Ra.sn * eaq.y);
-          x[1][c] = make_double2(Ra.sn * ap.x + Ra.cs * eaq.x, Ra.sn * ap.y + Ra.cs * eaq.y);
+        for (int u = 0; u < kJRows / kJT; u++) {
+          const int row = ta * kJRows + la + kJT * u;
+          if (row >= n) continue;
+          turn(Rb, wb, v[u][0], v[u][1], false);
+          __stcg(&V[(long)row * n + pb], v[u][0]);
+          __stcg(&V[(long)row * n + qb], v[u][1]);
         }
-        const double2 eb = make_double2(Rb.pr, -Rb.pi);
-#pragma unroll
-        for (int rw = 0; rw < 2; rw++) {
-          const double2 ap = x[rw][0], aq = x[rw][1];
-          const double2 eaq = make_double2(eb.x * aq.x - eb.y * aq.y, eb.x * aq.y + eb.y * aq.x);
-          x[rw][0] = make_double2(Rb.cs * ap.x - Rb.sn * eaq.x, Rb.cs * ap.y - Rb.sn * eaq.y);
-          x[rw][1] = make_double2(Rb.sn * ap.x + Rb.cs * eaq.x, Rb.sn * ap.y + Rb.cs * eaq.y);
-        }
-        if (w / half == w % half && !(Ra.cs == 1.0 && Ra.sn == 0.0)) {
-          x[0][1] = make_double2(0, 0);
-          x[1][0] = make_double2(0, 0);
-        }
-        A[(long)Ra.p * n + Rb.p] = x[0][0];
-        if (qb) A[(long)Ra.p * n + Rb.q] = x[0][1];
-        if (qa) A[(long)Ra.q * n + Rb.p] = x[1][0];
-        if (qa && qb) A[(long)Ra.q * n + Rb.q] = x[1][1];
-      } else {
-        const long w2 = w - nblk;
-        const Rot R = rot[w2 / n];
-        const int row = (int)(w2 % n);
-        if (R.q >= n) continue;
-        const double2 ap = V[(long)row * n + R.p], aq = V[(long)row * n + R.q];
-        const double2 e = make_double2(R.pr, -R.pi);
-        const double2 eaq = make_double2(e.x * aq.x - e.y * aq.y, e.x * aq.y + e.y * aq.x);
-        V[(long)row * n + R.p] = make_double2(R.cs * ap.x - R.sn * eaq.x, R.cs * ap.y - R.sn * eaq.y);
-        V[(long)row * n + R.q] = make_double2(R.sn * ap.x + R.cs * eaq.x, R.sn * ap.y + R.cs * eaq.y);
       }
     }
-    grid.sync();
+    gen += gridDim.x;
+    if (!grid_barrier(counter, gen)) {
+      if (tid == 0) off[2] = 1.0;
+      return;
+    }
   }
-  // off-diagonal Frobenius norm and diagonal norm: per-warp partials
-  // (off[2 + 2 w], off[3 + 2 w]) summed by warp 0 of block 0 in a fixed order,
-  // so that the sweep count is the same on every run
+  // off-diagonal Frobenius norm and diagonal norm: per-CTA partials summed by
+  // CTA 0 in a fixed order, so that the sweep count is the same on every run
+  const double2 *A = ((m - 1) & 1) ? A1 : A0;
   double so = 0, sd = 0;
-  for (long e = tid; e < (long)n * n; e += nth) {
-    const double2 a = A[e];
-    const double v = a.x * a.x + a.y * a.y;
-    if (e / n == e % n) sd += v;
-    else so += v;
+  for (long e = blockIdx.x * (long)kJThreads + tid; e < (long)n * n; e += (long)gridDim.x * kJThreads) {
+    const double2 a = __ldcg(&A[e]);
+    const double t = a.x * a.x + a.y * a.y;
+    if (e / n == e % n) sd += t;
+    else so += t;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    so += __shfl_xor_sync(0xffffffffu, so, o);
-    sd += __shfl_xor_sync(0xffffffffu, sd, o);
-  }
-  const long nw = nth / 32, w = tid / 32;
-  if ((threadIdx.x & 31) == 0) {
-    off[2 + 2 * w] = so;
-    off[3 + 2 * w] = sd;
-  }
-  grid.sync();
-  if (blockIdx.x == 0 && threadIdx.x < 32) {
-    double to = 0, td = 0;
-    for (long i = threadIdx.x; i < nw; i += 32) {
-      to += off[2 + 2 * i];
-      td += off[3 + 2 * i];
-    }
+  __shared__ double ws[2][kJThreads / 32];
+  auto warp_sums = [&](double &x, double &y) {
     for (int o = 16; o > 0; o >>= 1) {
-      to += __shfl_xor_sync(0xffffffffu, to, o);
-      td += __shfl_xor_sync(0xffffffffu, td, o);
+      x += __shfl_xor_sync(0xffffffffu, x, o);
+      y += __shfl_xor_sync(0xffffffffu, y, o);
     }
-    if (threadIdx.x == 0) {
+  };
+  warp_sums(so, sd);
+  if ((tid & 31) == 0) {
+    ws[0][tid >> 5] = so;
+    ws[1][tid >> 5] = sd;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __stcg(&off[3 + 2 * blockIdx.x], ws[0][0] + ws[0][1]);
+    __stcg(&off[4 + 2 * blockIdx.x], ws[1][0] + ws[1][1]);
+  }
+  gen += gridDim.x;
+  if (!grid_barrier(counter, gen)) {
+    if (tid == 0) off[2] = 1.0;
+    return;
+  }
+  if (blockIdx.x == 0 && tid < 32) {
+    double to = 0, td = 0;
+    for (int i = tid; i < (int)gridDim.x; i += 32) {
+      to += __ldcg(&off[3 + 2 * i]);
+      td += __ldcg(&off[4 + 2 * i]);
+    }
+    warp_sums(to, td);
+    if (tid == 0) {
       off[0] = to;
       off[1] = td;
     }
@@ -351,41 +445,46 @@ __global__ void k_identity(double2 *V, int n)
 
 // eigen-decomposition of the Hermitian n x n matrix A (device, overwritten);
 // V (device, n x n) receives the eigenvectors as columns, w (host) the
-// eigenvalues in the order of V's columns
-int jacobi_eig_dev(fbse_ctx *c, double2 *A, double2 *V, int n, std::vector<double> &w)
+// eigenvalues in the order of V's columns.  real: A has no imaginary part
+int jacobi_eig_dev(fbse_ctx *c, double2 *A, double2 *V, int n, std::vector<double> &w, bool real)
 {
   const int m = n + (n & 1);
+  const void *kernel = real ? (const void *)k_jacobi_sweep<true> : (const void *)k_jacobi_sweep<false>;
   int dev = 0, nsm = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jacobi_sweep, 256, 0);
-  const long work = (long)(m / 2) * (m / 2) + (long)n * (m / 2);
-  long want = (work + 255) / 256;
-  int blocks = (int)std::min<long>(std::max<long>(1, want), (long)nsm * std::max(1, per_sm));
-  // rotation table, the two norms and their per-warp partials, kept in the
-  // context between calls
-  const size_t rot_bytes = (sizeof(Rot) * (m / 2 + 1) + 15) / 16 * 16;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kJThreads, 0);
+  const long T = (m / 2 + kJT - 1) / kJT, tiles = T * T + T * ((n + kJRows - 1) / kJRows);
+  // a tile per CTA, up to four CTAs per SM (more only lengthen the barrier)
+  const int blocks = (int)std::min<long>(std::max<long>(1, tiles), (long)nsm * std::min(4, std::max(1, per_sm)));
+  // the second buffer of A, the norms and their partials, the barrier's counter,
+  // kept in the context between calls
+  const size_t a_bytes = (size_t)n * n * sizeof(double2), off_bytes = (3 + 2 * (size_t)blocks) * sizeof(double);
   void *scratch = nullptr;
-  int rc = cached(c, kSlotJacobi, rot_bytes + (2 + 2 * (size_t)blocks * 8) * sizeof(double), &scratch);
+  int rc = cached(c, kSlotJacobi, a_bytes + off_bytes + 16, &scratch);
   if (rc) return rc;
-  Rot *rot = static_cast<Rot *>(scratch);
-  double *off = reinterpret_cast<double *>(static_cast<char *>(scratch) + rot_bytes);
+  double2 *A1 = static_cast<double2 *>(scratch), *cur = A, *other = A1;
+  double *off = reinterpret_cast<double *>(static_cast<char *>(scratch) + a_bytes);
+  unsigned *counter = reinterpret_cast<unsigned *>(off + 3 + 2 * blocks), count = 0;
+  FBSE_CUDA(c, cudaMemsetAsync(off, 0, off_bytes + 16, c->stream));
   FBSE_COUNT(1); k_identity<<<256, 256, 0, c->stream>>>(V, n);
-  double h[2] = {0, 0};
+  double h[3] = {0, 0, 0};
   bool conv = (n < 2);
   for (int sweep = 0; sweep < 60 && !conv; sweep++) {
-    void *args[] = {&A, &V, &n, (void *)&m, &rot, &off};
     int mm = m;
-    args[3] = &mm;
-    FBSE_COUNT(1); if (cudaLaunchCooperativeKernel((void *)k_jacobi_sweep, blocks, 256, args, 0, c->stream) != cudaSuccess) {
+    void *args[] = {&cur, &other, &V, &n, &mm, &counter, &count, &off};
+    FBSE_COUNT(1); if (cudaLaunchCooperativeKernel(kernel, blocks, kJThreads, args, 0, c->stream) != cudaSuccess) {
       rc = set_err(c, FBSE_ERR_CUDA, std::string("jacobi launch: ") + cudaGetErrorString(cudaGetLastError()));
       break;
     }
-    if (cudaMemcpyAsync(h, off, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
+    count += (unsigned)m * (unsigned)blocks;  // m - 1 rounds and the norms
+    if ((m - 1) & 1) std::swap(cur, other);
+    if (cudaMemcpyAsync(h, off, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) {
       rc = set_err(c, FBSE_ERR_CUDA, "jacobi sweep");
       break;
     }
+    if (h[2] != 0) { rc = set_err(c, FBSE_ERR_NOCONV, "jacobi: a grid barrier timed out"); break; }
     if (!(h[0] == h[0])) { rc = set_err(c, FBSE_ERR_NAN, "jacobi: NaN in matrix"); break; }
     if (h[0] <= 1e-30 * h[1] || h[0] < 1e-300) conv = true;
   }
@@ -393,7 +492,7 @@ int jacobi_eig_dev(fbse_ctx *c, double2 *A, double2 *V, int n, std::vector<doubl
   if (!rc) {
     // only the diagonal is needed on the host: one strided copy (pitch n + 1)
     std::vector<double2> d((size_t)n);
-    if (cudaMemcpy2DAsync(d.data(), sizeof(double2), A, (size_t)(n + 1) * sizeof(double2), sizeof(double2), (size_t)n,
+    if (cudaMemcpy2DAsync(d.data(), sizeof(double2), cur, (size_t)(n + 1) * sizeof(double2), sizeof(double2), (size_t)n,
                           cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
       rc = set_err(c, FBSE_ERR_CUDA, "jacobi download");
@@ -569,19 +668,25 @@ __global__ void __launch_bounds__(256, PART == 2 ? 1 : 2) k_rotate(const double 
   }
 }
 
-__global__ void k_sum_rot(const double *__restrict__ part, int nblk, int k, double *__restrict__ out)
+// out[3 s + q] = the sum of the rotation's per-tile partials, one CTA per state
+// (a thread's tiles in order, then a fixed tree); one thread per state walked the
+// 10^4 partials of 86^3 in 3.0 ms
+__global__ void __launch_bounds__(128) k_sum_rot(const double *__restrict__ part, int nblk, int k, double *__restrict__ out)
 {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < k; s += gridDim.x * blockDim.x) {
-    double a = 0, b = 0, d = 0;
-    for (int q = 0; q < nblk; q++) {
-      a += part[((long)q * k + s) * 3];
-      b += part[((long)q * k + s) * 3 + 1];
-      d += part[((long)q * k + s) * 3 + 2];
-    }
-    out[3 * s] = a;
-    out[3 * s + 1] = b;
-    out[3 * s + 2] = d;
+  const int s = blockIdx.x;
+  double v[3] = {0, 0, 0};
+  for (int t = threadIdx.x; t < nblk; t += blockDim.x) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) v[q] += part[((long)t * k + s) * 3 + q];
   }
+  __shared__ double w[4][3];
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5][q] = v[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) out[3 * s + threadIdx.x] = (w[0][threadIdx.x] + w[1][threadIdx.x]) + (w[2][threadIdx.x] + w[3][threadIdx.x]);
 }
 
 __global__ void k_scale_copy(const double *__restrict__ src, double *__restrict__ dst, long stlen, long k,
@@ -644,38 +749,47 @@ template <typename T>
 static int gram_t(fbse_ctx *c, const double *A, const double *B, int n, long L, double2 *out, double scale,
                   double2 *part, int nchunk, long kchunk)
 {
-  if constexpr (sizeof(T) == 8) {
-    if (L >= kExactMin) {
-      const long ld = (c->is_complex + 1) * L;
-      const int rc = exact_nt(c, A, ld, n, B, ld, n, L, c->is_complex ? kExactConj : kExactReal, scale, out);
-      if (rc != FBSE_ERR_OOM) return rc;
-    }
-  }
-  const int nt = (n + 63) / 64;
-  dim3 g(nt * (nt + 1) / 2, 1, nchunk);
-  // resident CTAs per SM: one (no register cap) or two (a cap of 128
-  // registers, which spills the FP32 path's float-float accumulators a
-  // little); the same sums either way, so the autotuner picks by time
-  auto launch = [&](long v) -> int {
-    if (c->is_complex) {
-      if (v == 2) k_gram<T, true, 2><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
-      else k_gram<T, true, 1><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
-    } else {
-      if (v == 2) k_gram<T, false, 2><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
-      else k_gram<T, false, 1><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
-    }
-    return launch_status(c);
+  auto sums = [&]() -> int {
+    k_sum_partials<<<256, 256, 0, c->stream>>>(part, nchunk, (long)n * n, scale, out);
+    FBSE_CHECK_LAUNCH(c);
+    return FBSE_OK;
   };
-  long minb = 1;
-  const std::string prob = std::string(sizeof(T) == 4 ? "fp32" : "fp64") + (c->is_complex ? " complex" : " real") +
-                           " n=" + std::to_string(n) + " L=" + std::to_string(L);
-  int rc = autotune(c, "gram CTAs per SM", prob, {1, 2}, launch, &minb);
-  if (rc) return rc;
-  if ((rc = launch(minb))) return rc;
-  FBSE_COUNT(1);
-  k_sum_partials<<<256, 256, 0, c->stream>>>(part, nchunk, (long)n * n, scale, out);
-  FBSE_CHECK_LAUNCH(c);
-  return FBSE_OK;
+  if constexpr (sizeof(T) == 8) {
+    // FP64 sums run at the FP64 pipe's rate whatever the tile, so 32 x 32 tiles, which
+    // give more CTAs (the same sums as 64 x 64): 10.0 -> 7.5 ms for 128 real states of 133380 points (5.4 ms of FP64 pipe).  The exact
+    // products of exactgemm.cu take 0.2 ms, but their last bits differ (see the
+    // caller).
+    const int nt = (n + 63) / 64;
+    const dim3 g(4 * nt * (nt + 1) / 2, 1, nchunk);
+    if (c->is_complex) k_gram<T, true, 2, 32><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
+    else k_gram<T, false, 2, 32><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
+    FBSE_CHECK_LAUNCH(c);
+    return sums();
+  } else {
+    const int nt = (n + 63) / 64;
+    dim3 g(nt * (nt + 1) / 2, 1, nchunk);
+    // resident CTAs per SM: one (no register cap) or two (a cap of 128
+    // registers, which spills the FP32 path's float-float accumulators a
+    // little); the same sums either way, so the autotuner picks by time
+    auto launch = [&](long v) -> int {
+      if (c->is_complex) {
+        if (v == 2) k_gram<T, true, 2><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
+        else k_gram<T, true, 1><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
+      } else {
+        if (v == 2) k_gram<T, false, 2><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
+        else k_gram<T, false, 1><<<g, 256, 0, c->stream>>>(A, B, n, L, kchunk, part);
+      }
+      return launch_status(c);
+    };
+    long minb = 1;
+    const std::string prob = std::string("fp32") + (c->is_complex ? " complex" : " real") +
+                             " n=" + std::to_string(n) + " L=" + std::to_string(L);
+    int rc = autotune(c, "gram CTAs per SM", prob, {1, 2}, launch, &minb);
+    if (rc) return rc;
+    if ((rc = launch(minb))) return rc;
+    FBSE_COUNT(1);
+    return sums();
+  }
 }
 
 // default overlap cut of the mixed path, relative to the largest eigenvalue.
@@ -717,13 +831,15 @@ static int ortho_diag_sigma_t(fbse_ctx *c, double *psitot, long n_, long *n_kept
     rc = set_err(c, FBSE_ERR_OOM, "ortho/diag scratch");
     return false;
   };
-  // Ritz vectors of close pairs follow the rounding of the FP32 H psi: a change of
-  // 1e-7 in it moved vectors by up to 2e-3 (128 states, 86^3), so this step keeps
-  // one set of FFT kernels whatever H psi itself uses, and with it the vectors of
-  // earlier runs.  It applies H once per state, the filter thousands of times.
+  // The Ritz vectors follow the last bits of this step's sums: close pairs by their
+  // size (FP32: a change of 1e-7 in H psi moved vectors by up to 2e-3, 128 states of
+  // 86^3), and every complex vector by its phase, which Jacobi takes from elements
+  // that have almost vanished.  So this step keeps one set of H psi kernels and one
+  // sum order whatever H psi itself uses, and with them the vectors of earlier runs.
+  // It applies H once per state, the filter thousands of times.
   struct Steady {
     fbse_ctx *c;
-    explicit Steady(fbse_ctx *c_) : c(c_) { c->steady = kMixed; }
+    explicit Steady(fbse_ctx *c_) : c(c_) { c->steady = 1; }
     ~Steady() { c->steady = 0; }
   } steady(c);
   do {
@@ -778,7 +894,7 @@ static int ortho_diag_sigma_t(fbse_ctx *c, double *psitot, long n_, long *n_kept
     }
     // 3. overlap eigen-decomposition
     std::vector<double> w;
-    if ((rc = jacobi_eig_dev(c, G, V, n, w))) break;
+    if ((rc = jacobi_eig_dev(c, G, V, n, w, !c->is_complex))) break;
     // 4. rank cutoff (ortho.c:68-75 keeps s_i/s_0 >= 1e-10); the overlap
     //    resolves l_i / l_max to the precision of its products and of the
     //    states (fbse_tuning.ritz_cut overrides the default)
@@ -807,7 +923,7 @@ static int ortho_diag_sigma_t(fbse_ctx *c, double *psitot, long n_, long *n_kept
     if ((rc = zgemm_dev(c, k, k, n, X, k, true, Tm, k, false, Hp, k))) break;  // Hp = X^H Tm (k x k)
     FBSE_COUNT(1); k_hermitize<<<64, 256, 0, c->stream>>>(Hp, k);
     std::vector<double> e;
-    if ((rc = jacobi_eig_dev(c, Hp, U, k, e))) break;
+    if ((rc = jacobi_eig_dev(c, Hp, U, k, e, !c->is_complex))) break;
     std::vector<int> perm(k);
     std::iota(perm.begin(), perm.end(), 0);
     std::sort(perm.begin(), perm.end(), [&](int a, int b) { return e[a] < e[b]; });
@@ -845,7 +961,7 @@ static int ortho_diag_sigma_t(fbse_ctx *c, double *psitot, long n_, long *n_kept
       else k_rotate<T, false, 2><<<gr, 256, 0, c->stream>>>(psitot, hpsi, n, L, Cm, k, Ed, rot, rpart);
     }
     FBSE_LAUNCH_OR_BREAK(c, rc);
-    FBSE_COUNT(1); k_sum_rot<<<(k + 127) / 128, 128, 0, c->stream>>>(rpart, nrb, k, rsum);
+    FBSE_COUNT(1); k_sum_rot<<<k, 128, 0, c->stream>>>(rpart, nrb, k, rsum);
     std::vector<double> hs(3 * k), hq(2 * (size_t)n);
     if (cudaMemcpyAsync(hs.data(), rsum, 3 * k * sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
         (kMixed && cudaMemcpyAsync(hq.data(), quad, 2 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost,
