@@ -97,25 +97,49 @@ __global__ void k_pot_kspace(int nx, int ny, int nz, double dkx, double dky, dou
 }
 
 // ---------------------------------------------------------------------------
-// pair densities rho[p][r] = sum_sigma conj(psi_x(r,sigma)) psi_y(r,sigma)
-// for a list of (x, y) state pairs (indices into psi_qp)
+// pair densities rho_xy[r] = sum_sigma conj(psi_x(r,sigma)) psi_y(r,sigma) of the
+// items' state pairs (x, y) into row d1 of D1, and rho_yx = conj(rho_xy) into row d2
+// of D2 unless d2 < 0.  The FP64 pipe bounds it (10 operations a point and pair), so
+// both orders of a pair, and the hole-electron densities of both exchange factors,
+// are formed once: 16 x 16 pairs of two-spinor states, 96^3, 1024 densities in FP32
+// 23.6 -> 12.0 ms.
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void k_pair_density(const double2 *__restrict__ psi, long nsg, long ngrid, int nspin,
-                               const int2 *__restrict__ pairs, int npairs, C<T> *__restrict__ rho)
+struct PairItem {
+  int x, y, d1, d2;
+};
+
+template <typename T, int NS>
+__global__ void __launch_bounds__(256) k_pair_density(const double2 *__restrict__ psi, long ngrid,
+                                                      const PairItem *__restrict__ items, C<T> *__restrict__ D1,
+                                                      C<T> *__restrict__ D2)
 {
-  const long total = (long)npairs * ngrid;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-    const int p = (int)(e / ngrid);
-    const long r = e - (long)p * ngrid;
-    const int2 xy = pairs[p];
-    double sr = 0.0, si = 0.0;
-    for (int s = 0; s < nspin; s++) {
-      const double2 a = psi[(long)xy.x * nsg + s * ngrid + r], b = psi[(long)xy.y * nsg + s * ngrid + r];
-      sr += a.x * b.x + a.y * b.y;  // conj(a) b
-      si += a.x * b.y - a.y * b.x;
+  constexpr int U = 4;  // points per thread: loads of several in flight
+  const PairItem it = items[blockIdx.y];
+  const double2 *px = psi + (long)it.x * NS * ngrid, *py = psi + (long)it.y * NS * ngrid;
+  const long r0 = (long)blockIdx.x * (256 * U) + threadIdx.x;
+  double2 a[U][NS], b[U][NS];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const long r = r0 + 256 * u;
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+      a[u][s] = r < ngrid ? px[s * ngrid + r] : make_double2(0, 0);
+      b[u][s] = r < ngrid ? py[s * ngrid + r] : make_double2(0, 0);
     }
-    rho[e] = mk<T>((T)sr, (T)si);
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const long r = r0 + 256 * u;
+    if (r >= ngrid) return;
+    double sr = 0.0, si = 0.0;
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+      sr += a[u][s].x * b[u][s].x + a[u][s].y * b[u][s].y;  // conj(a) b
+      si += a[u][s].x * b[u][s].y - a[u][s].y * b[u][s].x;
+    }
+    const T tr = (T)sr, ti = (T)si;
+    D1[(long)it.d1 * ngrid + r] = mk<T>(tr, ti);
+    if (it.d2 >= 0) D2[(long)it.d2 * ngrid + r] = mk<T>(tr, -ti);
   }
 }
 
@@ -233,16 +257,17 @@ static int cgemm_nt(fbse_ctx *c, const C<T> *A, int ma, const C<T> *B, int nb, l
 }
 
 // scatter the (pair x pair) GEMM result into the n_xton x n_xton kernel:
-// direct: Kd[ibs][jbs] = G[(a,b)][(j,i)], ibs = a*nh + i, jbs = b*nh + j
+// direct: Kd[ibs][jbs] = G[row of (a,b)][(j,i)], ibs = a*nh + i, jbs = b*nh + j
 // exchange: Kx[ibs][jbs] = G[ibs][jbs]; only ibs >= jbs is kept
-__global__ void k_scatter_direct(const double2 *__restrict__ G, int ne, int nh, double2 *__restrict__ K)
+__global__ void k_scatter_direct(const double2 *__restrict__ G, int ne, int nh, const int *__restrict__ row,
+                                 double2 *__restrict__ K)
 {
   const long nx = (long)ne * nh;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < nx * nx; e += (long)gridDim.x * blockDim.x) {
     const long ibs = e / nx, jbs = e % nx;
     if (ibs < jbs) { K[e] = make_double2(0, 0); continue; }
     const long a = ibs / nh, i = ibs % nh, b = jbs / nh, j = jbs % nh;
-    K[e] = G[(a * ne + b) * ((long)nh * nh) + (j * nh + i)];
+    K[e] = G[(long)row[a * ne + b] * ((long)nh * nh) + (j * nh + i)];
   }
 }
 
@@ -252,26 +277,46 @@ __global__ void k_lower_only(double2 *K, long n)
     if (e / n < e % n) K[e] = make_double2(0, 0);
 }
 
-// pair densities for a list of (x, y) pairs into dst[p][r]; with conv set, each
-// density is convolved with that k-space potential (hartree, bse_cplx/hartree.c)
-// in batches: wk holds 2 x batch grids (densities, FFT scratch)
+// pair densities of items [i0, i1) (uploaded in ditems)
 template <typename T>
-static int conv_batches(fbse_ctx *c, const double *psi_qp, const std::vector<int2> &pairs, C<T> *dst, C<T> *wk,
-                        long batch, int2 *dpairs, const double2 *conv)
+static int densities(fbse_ctx *c, const double *psi_qp, const PairItem *ditems, long i0, long i1, C<T> *D1, C<T> *D2)
+{
+  const unsigned gx = (unsigned)((c->ngrid + 1023) / 1024);
+  for (long i = i0; i < i1; i += 65535) {
+    const dim3 g(gx, (unsigned)std::min<long>(65535, i1 - i));
+    if (c->nspin == 2)
+      k_pair_density<T, 2><<<g, 256, 0, c->stream>>>((const double2 *)psi_qp, c->ngrid, ditems + i, D1, D2);
+    else
+      k_pair_density<T, 1><<<g, 256, 0, c->stream>>>((const double2 *)psi_qp, c->ngrid, ditems + i, D1, D2);
+    FBSE_CHECK_LAUNCH(c);
+  }
+  return FBSE_OK;
+}
+
+// the densities of the items' d1 rows (and d2 rows when they lie in the same list,
+// both: D2 null), convolved with the k-space potential conv (hartree,
+// bse_cplx/hartree.c) into dst rows 0 .. rows - 1, in batches of rows: wk holds 2 x
+// batch grids (densities, FFT scratch).  Items are sorted by d1, an item's rows lie
+// in one batch, and their numbers are made relative to it here.
+template <typename T>
+static int conv_batches(fbse_ctx *c, const double *psi_qp, std::vector<PairItem> items, long rows, C<T> *dst, C<T> *wk,
+                        long batch, PairItem *ditems, const double2 *conv, C<T> *D2)
 {
   const long N = c->ngrid;
-  const long nsg = (long)c->nspin * N;
-  FBSE_CUDA(c, cudaMemcpyAsync(dpairs, pairs.data(), pairs.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
-  for (long p0 = 0; p0 < (long)pairs.size(); p0 += batch) {
-    const int np = (int)std::min<long>(batch, (long)pairs.size() - p0);
-    C<T> *tgt = dst + p0 * N;
-    k_pair_density<T><<<gridn((long)np * N), 256, 0, c->stream>>>((const double2 *)psi_qp, nsg, N, c->nspin,
-                                                                     dpairs + p0, np, conv ? wk : tgt);
-    FBSE_CHECK_LAUNCH(c);
-    if (conv) {
-      const int r2 = conv_apply<T>(c, wk, tgt, wk + batch * N, np, conv);
-      if (r2) return r2;
-    }
+  for (PairItem &it : items) {
+    it.d1 = (int)(it.d1 % batch);
+    if (!D2 && it.d2 >= 0) it.d2 = (int)(it.d2 % batch);
+  }
+  FBSE_CUDA(c, cudaMemcpyAsync(ditems, items.data(), items.size() * sizeof(PairItem), cudaMemcpyHostToDevice, c->stream));
+  long i0 = 0;
+  for (long p0 = 0; p0 < rows; p0 += batch) {
+    const long np = std::min<long>(batch, rows - p0);
+    long i1 = i0 + 1;  // the next batch starts where d1 wraps
+    while (i1 < (long)items.size() && items[i1].d1 > items[i1 - 1].d1) i1++;
+    int rc = densities<T>(c, psi_qp, ditems, i0, i1, wk, D2 ? D2 : wk);
+    if (!rc) rc = conv_apply<T>(c, wk, dst + p0 * N, wk + batch * N, np, conv);
+    if (rc) return rc;
+    i0 = i1;
   }
   return FBSE_OK;
 }
@@ -283,9 +328,11 @@ static int eh_kernels_t(fbse_ctx *c, const double *psi_qp, long nh, long ne, lon
   const long N = c->ngrid;
   const long nx = ne * nh;
   int rc = FBSE_OK;
-  const long batch = std::max<long>(1, std::min<long>(64, (long)(2.0e9 / (N * sizeof(C<T>)))));
+  // rows per FFT batch, even so that both orders of a pair share a batch
+  const long batch = std::max<long>(2, std::min<long>(64, (long)(2.0e9 / (N * sizeof(C<T>)))) / 2 * 2);
   C<T> *P = nullptr, *Q = nullptr, *wk = nullptr;
-  int2 *dpairs = nullptr;
+  PairItem *ditems = nullptr;
+  int *drow = nullptr;
   double2 *G = nullptr;
   const long maxrows = std::max(ne * ne, std::max(nh * nh, nx));
   auto fail = [&](const char *m) { cudaGetLastError(); rc = set_err(c, FBSE_ERR_OOM, m); };
@@ -298,32 +345,51 @@ static int eh_kernels_t(fbse_ctx *c, const double *psi_qp, long nh, long ne, lon
   if (!get(&P, (size_t)maxrows * N * sizeof(C<T>))) fail("bse pair densities");
   else if (!get(&Q, (size_t)maxrows * N * sizeof(C<T>))) fail("bse pair densities");
   else if (!get(&wk, (size_t)2 * batch * N * sizeof(C<T>))) fail("bse fft scratch");
-  else if (!get(&dpairs, (size_t)maxrows * sizeof(int2))) fail("bse pairs");
+  else if (!get(&ditems, (size_t)maxrows * sizeof(PairItem)) || !get(&drow, (size_t)ne * ne * sizeof(int))) fail("bse pairs");
   else if (!get(&G, (size_t)(ne * ne) * (nh * nh) * sizeof(double2))) fail("bse G");
-  std::vector<int2> pr;
+  std::vector<PairItem> items;
+  std::vector<int> row((size_t)ne * ne);
   do {
     if (rc) break;
-    // ---- direct: P[(a,b)] = W * rho_ab, Q[(j,i)] = rho_ji
-    pr.clear();
+    // ---- direct: P[row(a,b)] = W * rho_ab, Q[(j,i)] = rho_ji; P's rows hold a pair's
+    // two orders one after the other
+    int next = 0;
     for (long a = 0; a < ne; a++)
-      for (long b = 0; b < ne; b++) pr.push_back(make_int2((int)(lumo + a), (int)(lumo + b)));
-    if ((rc = conv_batches<T>(c, psi_qp, pr, P, wk, batch, dpairs, (const double2 *)pot_scr))) break;
-    pr.clear();
+      for (long b = a; b < ne; b++) {
+        if (a == b) continue;
+        row[a * ne + b] = next;
+        row[b * ne + a] = next + 1;
+        items.push_back({(int)(lumo + a), (int)(lumo + b), next, next + 1});
+        next += 2;
+      }
+    for (long a = 0; a < ne; a++) {
+      row[a * ne + a] = next;
+      items.push_back({(int)(lumo + a), (int)(lumo + a), next++, -1});
+    }
+    if (cudaMemcpyAsync(drow, row.data(), row.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream) != cudaSuccess) {
+      rc = set_err(c, FBSE_ERR_CUDA, "bse pairs");
+      break;
+    }
+    if ((rc = conv_batches<T>(c, psi_qp, items, ne * ne, P, wk, batch, ditems, (const double2 *)pot_scr, nullptr))) break;
+    items.clear();
     for (long j = 0; j < nh; j++)
-      for (long i = 0; i < nh; i++) pr.push_back(make_int2((int)j, (int)i));
-    if ((rc = conv_batches<T>(c, psi_qp, pr, Q, wk, batch, dpairs, nullptr))) break;
+      for (long i = j; i < nh; i++)
+        items.push_back({(int)j, (int)i, (int)(j * nh + i), i == j ? -1 : (int)(i * nh + j)});
+    if (cudaMemcpyAsync(ditems, items.data(), items.size() * sizeof(PairItem), cudaMemcpyHostToDevice, c->stream) !=
+        cudaSuccess) {
+      rc = set_err(c, FBSE_ERR_CUDA, "bse pairs");
+      break;
+    }
+    if ((rc = densities<T>(c, psi_qp, ditems, 0, (long)items.size(), Q, Q))) break;
     if ((rc = cgemm_nt<T>(c, P, (int)(ne * ne), Q, (int)(nh * nh), N, c->dv, G))) break;
-    k_scatter_direct<<<gridn(nx * nx), 256, 0, c->stream>>>(G, (int)ne, (int)nh, (double2 *)direct);
+    k_scatter_direct<<<gridn(nx * nx), 256, 0, c->stream>>>(G, (int)ne, (int)nh, drow, (double2 *)direct);
     FBSE_LAUNCH_OR_BREAK(c, rc);
-    // ---- exchange: P[(a,i)] = v * rho_ai (ibs order), Q[(b,j)] = rho_jb (jbs order)
-    pr.clear();
+    // ---- exchange: P[(a,i)] = v * rho_ai (ibs order), Q[(a,i)] = rho_ia = conj(rho_ai)
+    items.clear();
     for (long a = 0; a < ne; a++)
-      for (long i = 0; i < nh; i++) pr.push_back(make_int2((int)(lumo + a), (int)i));
-    if ((rc = conv_batches<T>(c, psi_qp, pr, P, wk, batch, dpairs, (const double2 *)pot_bare))) break;
-    pr.clear();
-    for (long b = 0; b < ne; b++)
-      for (long j = 0; j < nh; j++) pr.push_back(make_int2((int)j, (int)(lumo + b)));
-    if ((rc = conv_batches<T>(c, psi_qp, pr, Q, wk, batch, dpairs, nullptr))) break;
+      for (long i = 0; i < nh; i++)
+        items.push_back({(int)(lumo + a), (int)i, (int)(a * nh + i), (int)(a * nh + i)});
+    if ((rc = conv_batches<T>(c, psi_qp, items, nx, P, wk, batch, ditems, (const double2 *)pot_bare, Q))) break;
     if ((rc = cgemm_nt<T>(c, P, (int)nx, Q, (int)nx, N, -c->dv, (double2 *)exchange))) break;
     k_lower_only<<<gridn(nx * nx), 256, 0, c->stream>>>((double2 *)exchange, nx);
     FBSE_LAUNCH_OR_BREAK(c, rc);
@@ -333,7 +399,8 @@ static int eh_kernels_t(fbse_ctx *c, const double *psi_qp, long nh, long ne, lon
   if (P) cudaFree(P);
   if (Q) cudaFree(Q);
   if (wk) cudaFree(wk);
-  if (dpairs) cudaFree(dpairs);
+  if (ditems) cudaFree(ditems);
+  if (drow) cudaFree(drow);
   if (G) cudaFree(G);
   return rc;
 }
