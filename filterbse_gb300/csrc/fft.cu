@@ -696,7 +696,8 @@ static bool two_axis_ok(fbse_ctx *c, int axis)
 template <typename T>
 static int launch_cols_any(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, bool kmul, const KinArgs &ka)
 {
-  if (two_axis_ok(c, axis)) return kmul ? two_z<T>(c, data, nblk, ka) : two_y<T>(c, data, nblk, inv);
+  if (two_axis_ok(c, axis))
+    return kmul ? two_z<T>(c, data, nblk, ka) : two_y<T>(c, data, data, nblk, inv ? 1 : 0, nullptr, nullptr, T(1), T(0));
   switch (fast_axis_ok(c, c->ax[axis].n) ? c->ax[axis].n : 0) {
     case 64: return launch_cols_fast_n<T, 64>(c, data, nblk, axis, inv, kmul, ka);
     case 128: return launch_cols_fast_n<T, 128>(c, data, nblk, axis, inv, kmul, ka);
@@ -736,13 +737,25 @@ template <typename T>
 static int launch_x_any(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, int epi, const C<T> *phi,
                         const T *pot, T ca, T cb)
 {
-  if (two_axis_ok(c, 0)) return two_x<T>(c, in, out, nblk, inv, phi, pot, ca, cb);
+  if (two_axis_ok(c, 0)) return two_x<T>(c, in, out, nblk, inv ? (epi ? 2 : 1) : 0, phi, pot, ca, cb);
   switch (fast_axis_ok(c, c->nx) ? c->nx : 0) {
     case 64: return launch_x_fast_n<T, 64>(c, in, out, nblk, inv, epi, phi, pot, ca, cb);
     case 128: return launch_x_fast_n<T, 128>(c, in, out, nblk, inv, epi, phi, pot, ca, cb);
     case 256: return launch_x_fast_n<T, 256>(c, in, out, nblk, inv, epi, phi, pot, ca, cb);
     default: return launch_x<T>(c, in, out, nblk, inv, epi, phi, pot, ca, cb);
   }
+}
+
+// whole planes in shared memory (three passes over memory) or y and x lines (five) for
+// nblk blocks of the two-factor kernels.  FP32 passes are bound by memory and latency:
+// planes when they fit (8 blocks of 96^3 124 us, lines 131; 1 of 57 x 52 x 45 25 us,
+// lines 38).  FP64 passes are bound by the FP64 pipe, which a last wave of planes leaves
+// half idle: lines unless the planes fill whole waves of the 152 SMs (2 blocks of 96^3
+// 595 us, lines 455; 12 of 96^3 2598, lines 2458; 150 planes of 72 x 70 252, lines 292)
+template <typename T> static bool two_planes(fbse_ctx *c, long nblk)
+{
+  const long n = nblk * c->nz, waves = (n + 151) / 152;
+  return two_plane_smem<T>(c) <= (size_t)max_smem() && (sizeof(T) == 4 || n * 100 >= 97 * 152 * waves);
 }
 
 // out = a (F^-1 K F in + V in) + b in with K = the capped kinetic factor, or
@@ -756,14 +769,14 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
   const Stages sx = stages_of(c->ax[0]), sy = stages_of(c->ax[1]);
   const T *pot = with_v ? pot_of<T>(c) : nullptr;
   const bool fplane = fast_plane_ok<T>(c);
-  // a plane of two lengths that both have two factors (64, 128 and 256 do) when it fits
-  const bool tplane = !fplane && c->tune.fft_kernels == 0 && !c->steady && c->ax[0].P > 0 && c->ax[1].P > 0 &&
-                      two_plane_smem<T>(c) <= (size_t)max_smem();
+  // x and y both of two factors (64, 128 and 256 points are): whole planes in shared
+  // memory, or y and x lines with the same arithmetic in the same order
+  const bool both = !fplane && c->tune.fft_kernels == 0 && !c->steady && c->ax[0].P > 0 && c->ax[1].P > 0;
   const bool lines = two_axis_ok(c, 0) || two_axis_ok(c, 1);
   const bool plane = !lines && !sx.big && !sy.big && plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;
   // which of x and y the z pass meets in a two-factor transform's order
-  const bool xo = tplane || (!fplane && !plane && two_axis_ok(c, 0));
-  const bool yo = tplane || (!fplane && !plane && two_axis_ok(c, 1));
+  const bool xo = both || (!fplane && !plane && two_axis_ok(c, 0));
+  const bool yo = both || (!fplane && !plane && two_axis_ok(c, 1));
   const KinArgs ka = kin_args(c, kq, xo, yo);
   for (long b0 = 0; b0 < nblk; b0 += cb) {
     const long nb = (nblk - b0 < cb) ? nblk - b0 : cb;
@@ -774,10 +787,16 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
       if ((rc = launch_plane_fast<T>(c, ci, wk, nb, 0, nullptr, nullptr, T(1), T(0)))) return rc;
       if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, ka))) return rc;
       if ((rc = launch_plane_fast<T>(c, wk, co, nb, 1, ci, pot, (T)a, (T)b))) return rc;
-    } else if (tplane) {
+    } else if (both && two_planes<T>(c, nb)) {
       if ((rc = two_plane<T>(c, ci, wk, nb, false, nullptr, nullptr, T(1), T(0)))) return rc;
       if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, ka))) return rc;
       if ((rc = two_plane<T>(c, wk, co, nb, true, ci, pot, (T)a, (T)b))) return rc;
+    } else if (both) {
+      if ((rc = two_y<T>(c, ci, wk, nb, 0, nullptr, nullptr, T(1), T(0)))) return rc;
+      if ((rc = two_x<T>(c, wk, wk, nb, 0, nullptr, nullptr, T(1), T(0)))) return rc;
+      if ((rc = launch_cols_any<T>(c, wk, nb, 2, false, true, ka))) return rc;
+      if ((rc = two_x<T>(c, wk, wk, nb, 1, nullptr, nullptr, T(1), T(0)))) return rc;
+      if ((rc = two_y<T>(c, wk, co, nb, 2, ci, pot, (T)a, (T)b))) return rc;
     } else if (plane) {
       if ((rc = launch_plane<T>(c, ci, wk, nb, 0, nullptr, nullptr, T(1), T(0)))) return rc;
       if ((rc = launch_cols<T>(c, wk, nb, 2, false, true, ka))) return rc;

@@ -100,8 +100,10 @@ template <typename T> size_t two_plane_smem(const fbse_ctx *c);
 template <typename T>
 int two_plane(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T> *phi, const T *pot, T ca, T cb);
 template <typename T> int two_z(fbse_ctx *c, C<T> *data, long nblk, const KinArgs &ka);
-template <typename T> int two_y(fbse_ctx *c, C<T> *data, long nblk, bool inv);
+// mode 0: forward, 1: inverse, 2: inverse with the final out = ca (r + V phi) + cb phi
 template <typename T>
-int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T> *phi, const T *pot, T ca, T cb);
+int two_y(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, int mode, const C<T> *phi, const T *pot, T ca, T cb);
+template <typename T>
+int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, int mode, const C<T> *phi, const T *pot, T ca, T cb);
 
 }  // namespace fbse

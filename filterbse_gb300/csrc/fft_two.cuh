@@ -24,12 +24,13 @@
 // round trips and an integer division per element on such lengths, and lengths
 // with a prime above 8 take a direct sum per output.  Measured, H psi through
 // those kernels -> these:
-//   116 x 117 x 120, 4 spinors, FP32 (memory and latency bound)  2101 -> 408 us
-//   96^3, 4 spinors, FP32 (127 terms of a filter)                  742 -> 214 us
-//   96^3, 6 spinors, FP64 (FP64 pipe bound; projectors 1.9 ms)     5131 -> 3921 us
-//   57 x 52 x 45, 8 packed states, FP64 (radices 13, 19)           1911 -> 513 us
+//   116 x 117 x 120, 4 spinors, FP32 (memory and latency bound)  2101 -> 376 us
+//   96^3, 4 spinors, FP32 (127 terms of a filter)                  742 -> 164 us
+//   96^3, 6 spinors, FP64 (FP64 pipe bound; projectors 1.6 ms)     5131 -> 3794 us
+//   57 x 52 x 45, 8 packed states, FP64 (radices 13, 19)           1911 -> 477 us
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "fft_radix.cuh"
@@ -390,41 +391,52 @@ __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>:
   stage_a<T, BIG, false>(az, lines, lds, at, [&](int c, int z, C<T> v) { d[z * es + c] = exch<T>(v); });
 }
 
-// y lines of planes too large for shared memory: L consecutive x of one plane,
-// global memory to global memory, one exchange
-template <typename T, bool BIG, bool INV>
+// what a line pass does besides its transform
+enum LineMode { kForward, kInverse, kFinal };  // kFinal: inverse, then out = ca (r + V phi) + cb phi
+
+// y lines: L consecutive x of one plane, global memory to global memory, one exchange
+template <typename T, bool BIG, LineMode MODE>
 __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>::ctas)
-    k_two_y(C<T> *__restrict__ data, Axis<T> ay, int nx, int L, int ntile)
+    k_two_y(const C<T> *in, C<T> *out, Axis<T> ay, int nx, int L, int ntile, const C<T> *__restrict__ phi,
+            const T *__restrict__ pot, long ngrid, T ca, T cb)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C<T> *S = reinterpret_cast<C<T> *>(smem_raw);
   const long pl = blockIdx.x / ntile;
   const int x0 = (int)(blockIdx.x - pl * ntile) * L;
   const Div lines((unsigned)min(L, nx - x0));
-  C<T> *d = data + pl * nx * ay.n + x0;
-  auto ldg = [&](int c, int y) { return INV ? exch<T>(d[y * nx + c]) : d[y * nx + c]; };
-  auto stg = [&](int c, int y, C<T> v) { d[y * nx + c] = INV ? exch<T>(v) : v; };
+  const long off = pl * nx * ay.n + x0;
+  const C<T> *src = in + off;
+  C<T> *dst = out + off;
   auto at = [&](int c, int y) -> C<T> & { return S[y * L + c]; };
   auto lds = [&](int c, int y) { return S[y * L + c]; };
   auto sts = [&](int c, int y, C<T> v) { S[y * L + c] = v; };
-  if constexpr (!INV) {
-    stage_a<T, BIG, true>(ay, lines, ldg, at, sts);
+  if constexpr (MODE == kForward) {
+    stage_a<T, BIG, true>(ay, lines, [&](int c, int y) { return src[y * nx + c]; }, at, sts);
     __syncthreads();
-    stage_b<T, false>(ay, lines, lds, stg);
+    stage_b<T, false>(ay, lines, lds, [&](int c, int y, C<T> v) { dst[y * nx + c] = v; });
   } else {
-    stage_b<T, true>(ay, lines, ldg, sts);
+    stage_b<T, true>(ay, lines, [&](int c, int y) { return exch<T>(src[y * nx + c]); }, sts);
     __syncthreads();
-    stage_a<T, BIG, false>(ay, lines, lds, at, stg);
+    if constexpr (MODE == kInverse) {
+      stage_a<T, BIG, false>(ay, lines, lds, at, [&](int c, int y, C<T> v) { dst[y * nx + c] = exch<T>(v); });
+    } else {
+      const C<T> *ph = phi + off;
+      const T *V = pot ? pot + off % ngrid : nullptr;  // a plane lies inside one block
+      stage_a<T, BIG, false>(ay, lines, lds, at, [&](int c, int y, C<T> v) {
+        const int o = y * nx + c;
+        dst[o] = epilogue<T>(exch<T>(v), ph[o], V, o, ca, cb);
+      });
+    }
   }
 }
 
 // x lines: L contiguous lines through shared memory with an odd line stride
-// (coalesced copies, lanes on consecutive lines in the stages); INV ends with
-// out = ca (r + V phi) + cb phi
-template <typename T, bool BIG, bool INV>
+// (coalesced copies, lanes on consecutive lines in the stages)
+template <typename T, bool BIG, LineMode MODE>
 __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>::ctas)
-    k_two_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Axis<T> ax, Div dn, long nlines, int L,
-            const C<T> *__restrict__ phi, const T *__restrict__ pot, long ngrid, T ca, T cb)
+    k_two_x(const C<T> *in, C<T> *out, Axis<T> ax, Div dn, long nlines, int L, const C<T> *__restrict__ phi,
+            const T *__restrict__ pot, long ngrid, T ca, T cb)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C<T> *S = reinterpret_cast<C<T> *>(smem_raw);
@@ -440,25 +452,26 @@ __global__ void __launch_bounds__(LineShape<T, BIG>::threads, LineShape<T, BIG>:
   auto at = [&](int y, int x) -> C<T> & { return S[y * pitch + x]; };
   auto ldx = [&](int y, int x) { return S[y * pitch + x]; };
   auto stx = [&](int y, int x, C<T> v) { S[y * pitch + x] = v; };
-  C<T> *dst = out + off;
-  if constexpr (!INV) {
+  if constexpr (MODE == kForward) {
     stage_a<T, BIG, true>(ax, lines, ldx, at, stx);
     __syncthreads();
     stage_b<T, false>(ax, lines, ldx, stx);
-    __syncthreads();
-#pragma unroll 4
-    for (unsigned i = threadIdx.x; i < count; i += blockDim.x) dst[i] = S[i + dn(i) * (pitch - n)];
   } else {
     stage_b<T, true>(ax, lines, [&](int y, int x) { return exch<T>(S[y * pitch + x]); }, stx);
     __syncthreads();
     stage_a<T, BIG, false>(ax, lines, ldx, at, stx);
-    __syncthreads();
+  }
+  __syncthreads();
+  C<T> *dst = out + off;
 #pragma unroll 4
-    for (unsigned i = threadIdx.x; i < count; i += blockDim.x) {
-      const C<T> r = exch<T>(S[i + dn(i) * (pitch - n)]);
-      long g = off + i;  // the lines of a tile may lie in two blocks
-      dst[i] = epilogue<T>(r, phi[g], pot, pot ? g % ngrid : 0, ca, cb);
+  for (unsigned i = threadIdx.x; i < count; i += blockDim.x) {
+    C<T> r = S[i + dn(i) * (pitch - n)];
+    if (MODE != kForward) r = exch<T>(r);
+    if (MODE == kFinal) {
+      const long g = off + i;  // the lines of a tile may lie in two blocks
+      r = epilogue<T>(r, phi[g], pot, pot ? g % ngrid : 0, ca, cb);
     }
+    dst[i] = r;
   }
 }
 
@@ -551,7 +564,8 @@ template <typename T> int two_z(fbse_ctx *c, C<T> *data, long nblk, const KinArg
                 data, az, L, ntile, c->ngrid, ka);
 }
 
-template <typename T> int two_y(fbse_ctx *c, C<T> *data, long nblk, bool inv)
+template <typename T>
+int two_y(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, int mode, const C<T> *phi, const T *pot, T ca, T cb)
 {
   using namespace two;
   const Axis<T> ay = axis_of<T>(c->ax[1]);
@@ -560,13 +574,16 @@ template <typename T> int two_y(fbse_ctx *c, C<T> *data, long nblk, bool inv)
   const size_t smem = (size_t)ay.n * L * sizeof(C<T>);
   const bool big = ay.Q > 16;
   const int th = round32(line_threads(c->ax[1]) * L, 64, big ? LineShape<T, true>::threads : LineShape<T, false>::threads);
-  auto go = [&](auto k) { return launch(c, k, nblk * c->nz * ntile, th, smem, data, ay, (int)c->nx, L, ntile); };
-  if (big) return inv ? go(k_two_y<T, true, true>) : go(k_two_y<T, true, false>);
-  return inv ? go(k_two_y<T, false, true>) : go(k_two_y<T, false, false>);
+  auto go = [&](auto k) {
+    return launch(c, k, nblk * c->nz * ntile, th, smem, in, out, ay, (int)c->nx, L, ntile, phi, pot, c->ngrid, ca, cb);
+  };
+  if (mode == kForward) return big ? go(k_two_y<T, true, kForward>) : go(k_two_y<T, false, kForward>);
+  if (mode == kInverse) return big ? go(k_two_y<T, true, kInverse>) : go(k_two_y<T, false, kInverse>);
+  return big ? go(k_two_y<T, true, kFinal>) : go(k_two_y<T, false, kFinal>);
 }
 
 template <typename T>
-int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T> *phi, const T *pot, T ca, T cb)
+int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, int mode, const C<T> *phi, const T *pot, T ca, T cb)
 {
   using namespace two;
   const Axis<T> ax = axis_of<T>(c->ax[0]);
@@ -579,8 +596,9 @@ int two_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, const C<T
   auto go = [&](auto k) {
     return launch(c, k, (nlines + L - 1) / L, th, smem, in, out, ax, dn, nlines, L, phi, pot, c->ngrid, ca, cb);
   };
-  if (big) return inv ? go(k_two_x<T, true, true>) : go(k_two_x<T, true, false>);
-  return inv ? go(k_two_x<T, false, true>) : go(k_two_x<T, false, false>);
+  if (mode == kForward) return big ? go(k_two_x<T, true, kForward>) : go(k_two_x<T, false, kForward>);
+  if (mode == kInverse) return big ? go(k_two_x<T, true, kInverse>) : go(k_two_x<T, false, kInverse>);
+  return big ? go(k_two_x<T, true, kFinal>) : go(k_two_x<T, false, kFinal>);
 }
 
 }  // namespace fbse

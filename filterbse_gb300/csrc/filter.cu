@@ -370,43 +370,42 @@ __global__ void __launch_bounds__(256) k_dots(const C<T> *__restrict__ x, const 
   }
 }
 
+// out[2 st + q] = the sum of state st's nb partials: a warp per state, each lane its
+// partials in order, then a fixed tree (one thread walking 64 of them took 9 us)
 __global__ void k_dots_final(const double *__restrict__ part, int nb, long nstates, double *__restrict__ out)
 {
-  for (long st = blockIdx.x * (long)blockDim.x + threadIdx.x; st < nstates; st += (long)gridDim.x * blockDim.x) {
-    double a0 = 0, a1 = 0;
-    for (int b = 0; b < nb; b++) { a0 += part[(st * nb + b) * 2]; a1 += part[(st * nb + b) * 2 + 1]; }
+  const long st = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (st >= nstates) return;
+  double a0 = 0, a1 = 0;
+  for (int b = lane; b < nb; b += 32) { a0 += part[(st * nb + b) * 2]; a1 += part[(st * nb + b) * 2 + 1]; }
+  for (int o = 16; o > 0; o >>= 1) {
+    a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+  }
+  if (lane == 0) {
     out[2 * st] = a0;
     out[2 * st + 1] = a1;
   }
 }
 
-// out_dev: 2 doubles per state (second used by mode 2)
-template <typename T>
-int state_dots_dev(fbse_ctx *c, const C<T> *x, const C<T> *y, long nstates, long len, int mode, double *out_dev)
-{
-  const size_t need = (size_t)nstates * kRedBlocks * 2 * sizeof(double);
-  int rc = ensure(c, (void **)&c->red, &c->red_bytes, need);
-  if (rc) return rc;
-  if (nstates > 65535) return set_err(c, FBSE_ERR_UNSUPPORTED, "too many states for one reduction");
-  dim3 g(kRedBlocks, (unsigned)nstates);
-  k_dots<T><<<g, 256, 0, c->stream>>>(x, y, len, mode, c->red);
-  FBSE_CHECK_LAUNCH(c);
-  k_dots_final<<<(unsigned)((nstates + 127) / 128), 128, 0, c->stream>>>(c->red, kRedBlocks, nstates, out_dev);
-  FBSE_CHECK_LAUNCH(c);
-  return FBSE_OK;
-}
-
+// 2 doubles per state to the host (second used by mode 2); the sums sit behind the
+// partials in the context's reduction buffer
 template <typename T>
 int state_dots(fbse_ctx *c, const C<T> *x, const C<T> *y, long nstates, long len, double *out_host, int mode)
 {
-  double *d = nullptr;
-  if (cudaMalloc(&d, nstates * 2 * sizeof(double)) != cudaSuccess) return set_err(c, FBSE_ERR_OOM, "dots");
-  int rc = state_dots_dev<T>(c, x, y, nstates, len, mode, d);
-  if (!rc && cudaMemcpyAsync(out_host, d, nstates * 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess)
-    rc = set_err(c, FBSE_ERR_CUDA, "dots download");
-  if (!rc && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = set_err(c, FBSE_ERR_CUDA, "dots sync");
-  cudaFree(d);
-  return rc;
+  int rc = ensure(c, (void **)&c->red, &c->red_bytes, (size_t)nstates * (kRedBlocks + 1) * 2 * sizeof(double));
+  if (rc) return rc;
+  if (nstates > 65535) return set_err(c, FBSE_ERR_UNSUPPORTED, "too many states for one reduction");
+  double *sums = c->red + nstates * kRedBlocks * 2;
+  dim3 g(kRedBlocks, (unsigned)nstates);
+  k_dots<T><<<g, 256, 0, c->stream>>>(x, y, len, mode, c->red);
+  FBSE_CHECK_LAUNCH(c);
+  k_dots_final<<<(unsigned)((nstates + 3) / 4), 128, 0, c->stream>>>(c->red, kRedBlocks, nstates, sums);
+  FBSE_CHECK_LAUNCH(c);
+  if (d2h(c->stream, out_host, sums, nstates * 2 * sizeof(double)) != cudaSuccess)
+    return set_err(c, FBSE_ERR_CUDA, "dots download");
+  return FBSE_OK;
 }
 template int state_dots<float>(fbse_ctx *, const C<float> *, const C<float> *, long, long, double *, int);
 template int state_dots<double>(fbse_ctx *, const C<double> *, const C<double> *, long, long, double *, int);
@@ -452,7 +451,7 @@ int normalize_all(fbse_ctx *c, double *psitot, long n, double *norms)
   std::vector<double> h(2 * n), f(n);
   do {
     FBSE_COUNT(2); k_sumsq<<<dim3(kRedBlocks, (unsigned)n), 256, 0, c->stream>>>(psitot, stlen, c->red);
-    k_dots_final<<<(unsigned)((n + 127) / 128), 128, 0, c->stream>>>(c->red, kRedBlocks, n, d);
+    k_dots_final<<<(unsigned)((n + 3) / 4), 128, 0, c->stream>>>(c->red, kRedBlocks, n, d);
     if (cudaMemcpyAsync(h.data(), d, n * 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) { rc = set_err(c, FBSE_ERR_CUDA, "norm reduction"); break; }
     for (long i = 0; i < n; i++) {
@@ -527,12 +526,65 @@ int energy_all(fbse_ctx *c, const double *psitot, long n, double *ene, double *s
 // ---------------------------------------------------------------------------
 // spectrum range (energy.c:169-379, iterative branch)
 // ---------------------------------------------------------------------------
+// y = s (a y + b x), with partials of |y|^2 (part[block]); a = 0 does not read y
+constexpr int kRangeBlocks = 304;
 template <typename T>
-__global__ void k_axpby(C<T> *__restrict__ y, const C<T> *__restrict__ x, long len, double a, double b)
-{  // y = a*y + b*x
+__global__ void __launch_bounds__(256) k_range_step(C<T> *__restrict__ y, const C<T> *__restrict__ x, long len, double a,
+                                                    double b, double s, double *__restrict__ part)
+{
+  double n2 = 0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < len; i += (long)gridDim.x * blockDim.x) {
-    C<T> v = y[i], u = x[i];
-    y[i] = mk<T>((T)(a * v.x + b * u.x), (T)(a * v.y + b * u.y));
+    const C<T> u = x[i];
+    double re = b * u.x, im = b * u.y;
+    if (a != 0.0) {
+      const C<T> v = y[i];
+      re = a * v.x + re;
+      im = a * v.y + im;
+    }
+    const C<T> w = mk<T>((T)(s * re), (T)(s * im));
+    y[i] = w;
+    n2 += (double)w.x * w.x + (double)w.y * w.y;
+  }
+  __shared__ double r[8];
+  for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+  if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = n2;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    n2 = 0;
+    for (int w = 0; w < 8; w++) n2 += r[w];
+    part[blockIdx.x] = n2;
+  }
+}
+
+// partials of <x|h> (real part) and |h|^2: part[2 block], part[2 block + 1]
+template <typename T>
+__global__ void __launch_bounds__(256) k_range_dots(const C<T> *__restrict__ x, const C<T> *__restrict__ h, long len,
+                                                    double *__restrict__ part)
+{
+  double e = 0, n2 = 0;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < len; i += (long)gridDim.x * blockDim.x) {
+    const C<T> u = x[i], v = h[i];
+    e += (double)u.x * v.x + (double)u.y * v.y;
+    n2 += (double)v.x * v.x + (double)v.y * v.y;
+  }
+  __shared__ double r[8][2];
+  for (int o = 16; o > 0; o >>= 1) {
+    e += __shfl_xor_sync(0xffffffffu, e, o);
+    n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    r[threadIdx.x >> 5][0] = e;
+    r[threadIdx.x >> 5][1] = n2;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    e = n2 = 0;
+    for (int w = 0; w < 8; w++) {
+      e += r[w][0];
+      n2 += r[w][1];
+    }
+    part[2 * blockIdx.x] = e;
+    part[2 * blockIdx.x + 1] = n2;
   }
 }
 
@@ -555,9 +607,23 @@ static int energy_range_t(fbse_ctx *c, long seed, long max_iter, double *emin_ou
   if (cudaMalloc(&hd, len * 2 * sizeof(double)) != cudaSuccess) { cudaFree(buf); return set_err(c, FBSE_ERR_OOM, "energy range"); }
   C<T> *phi = buf, *h = buf + len;
   std::vector<double> host(2 * len);
-  double dd[2];
   int rc = FBSE_OK;
   long it_total = 0;
+  // Each iteration needs its scalars on the host once: the state is kept
+  // unnormalised, u, with its norm known from the kernel that wrote it, so that one
+  // kernel steps (scaling by the norm of the state before), H is applied, one kernel
+  // forms <u|Hu> and |Hu|^2, and both kernels write their partial sums straight into
+  // pinned host memory: one synchronisation.  (Two rounds of partial sums, final sums,
+  // allocations and copies before: 236 us an iteration of 44^3 FP64 spinors, 166 now.)
+  double *sums = nullptr;  // [kRangeBlocks] |u|^2, [kRangeBlocks][2] <u|Hu>, |Hu|^2
+  if (cudaMallocHost(&sums, 3 * kRangeBlocks * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(buf);
+    cudaFree(hd);
+    return set_err(c, FBSE_ERR_OOM, "energy range");
+  }
+  const int nb = (int)std::min<long>(kRangeBlocks, (len + 1023) / 1024);
+  double u2 = 1, uhu = 0, h2 = 0;  // |u|^2, <u|Hu>, |Hu|^2, without dv
   auto draw = [&](void) -> int {
     for (int s = 0; s < c->nspin; s++) seed = fbse_host_init_psi(host.data() + 2 * s * c->ngrid, seed, c->ngrid, c->is_complex, c->dv);
     if (cudaMemcpyAsync(hd, host.data(), len * 2 * sizeof(double), cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
@@ -566,21 +632,33 @@ static int energy_range_t(fbse_ctx *c, long seed, long max_iter, double *emin_ou
     FBSE_CHECK_LAUNCH(c);
     return FBSE_OK;
   };
+  // u <- s (a u + b Hu), Hu, and the three sums
+  auto step = [&](double a, double b, double s) -> int {
+    k_range_step<T><<<nb, 256, 0, c->stream>>>(phi, h, len, a, b, s, sums);
+    FBSE_CHECK_LAUNCH(c);
+    int r = hpsi_apply<T>(c, phi, h, 1, 1.0, 0.0);
+    if (r) return r;
+    k_range_dots<T><<<nb, 256, 0, c->stream>>>(phi, h, len, sums + kRangeBlocks);
+    FBSE_CHECK_LAUNCH(c);
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, FBSE_ERR_CUDA, "energy range");
+    u2 = uhu = h2 = 0;
+    for (int i = 0; i < nb; i++) {
+      u2 += sums[i];
+      uhu += sums[kRangeBlocks + 2 * i];
+      h2 += sums[kRangeBlocks + 2 * i + 1];
+    }
+    return FBSE_OK;
+  };
   do {
     // ---- E_min: phi <- normalize(phi - tau H phi)   (energy.c:221-271)
     if ((rc = draw())) break;
-    double tau = 0.05, emin = 10.0, old = 0.0;
+    double tau = 0.05, emin = 10.0, old = 0.0, s = 1.0;
     if ((rc = hpsi_apply<T>(c, phi, h, 1, 1.0, 0.0))) break;
     for (long i = 0; std::fabs((emin - old) / emin) > 1.0e-6 && i < max_iter; i++) {
-      // h holds H phi_i
-      FBSE_COUNT(1); k_axpby<T><<<grid_for(len), 256, 0, c->stream>>>(phi, h, len, 1.0, -tau);
-      if ((rc = state_dots<T>(c, phi, nullptr, 1, len, dd, 0))) break;
-      const double nrm = std::sqrt(dd[0] * c->dv);
-      FBSE_COUNT(1); k_axpby<T><<<grid_for(len), 256, 0, c->stream>>>(phi, phi, len, 1.0 / nrm, 0.0);
-      if ((rc = hpsi_apply<T>(c, phi, h, 1, 1.0, 0.0))) break;
-      if ((rc = state_dots<T>(c, phi, h, 1, len, dd, 1))) break;
+      if ((rc = step(1.0, -tau, s))) break;
+      s = 1.0 / std::sqrt(u2 * c->dv);
       old = emin;
-      emin = dd[0] * c->dv;
+      emin = uhu / u2;
       if (i > 5 && (emin - old) > 0) tau -= 0.025;  // energy.c:262-269
       it_total++;
     }
@@ -590,14 +668,15 @@ static int energy_range_t(fbse_ctx *c, long seed, long max_iter, double *emin_ou
     double emax = 0.1;
     old = 0.0;
     if ((rc = hpsi_apply<T>(c, phi, h, 1, 1.0, 0.0))) break;
+    k_range_dots<T><<<nb, 256, 0, c->stream>>>(phi, h, len, sums + kRangeBlocks);
+    FBSE_LAUNCH_OR_BREAK(c, rc);
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) { rc = set_err(c, FBSE_ERR_CUDA, "energy range"); break; }
+    h2 = 0;
+    for (int i = 0; i < nb; i++) h2 += sums[kRangeBlocks + 2 * i + 1];
     for (long i = 0; std::fabs((emax - old) / emax) > 1.0e-6 && i < max_iter; i++) {
-      if ((rc = state_dots<T>(c, h, nullptr, 1, len, dd, 0))) break;
-      const double nrm = std::sqrt(dd[0] * c->dv);
-      FBSE_COUNT(1); k_axpby<T><<<grid_for(len), 256, 0, c->stream>>>(phi, h, len, 0.0, 1.0 / nrm);
-      if ((rc = hpsi_apply<T>(c, phi, h, 1, 1.0, 0.0))) break;
-      if ((rc = state_dots<T>(c, phi, h, 1, len, dd, 1))) break;
+      if ((rc = step(0.0, 1.0, 1.0 / std::sqrt(h2 * c->dv)))) break;
       old = emax;
-      emax = dd[0] * c->dv;
+      emax = uhu / u2;
       it_total++;
     }
     if (rc) break;
@@ -606,6 +685,7 @@ static int energy_range_t(fbse_ctx *c, long seed, long max_iter, double *emin_ou
     if (iters) *iters = it_total;
   } while (0);
   cudaStreamSynchronize(c->stream);
+  cudaFreeHost(sums);
   cudaFree(buf);
   cudaFree(hd);
   return rc;
