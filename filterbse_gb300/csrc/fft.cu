@@ -263,33 +263,82 @@ __device__ __forceinline__ void pass_reg(C<T> *buf, int es, int ls, int n, int L
 }
 
 // a pass with a radix above the register limit: direct DFT from buf into a
-// scratch of L lines (element i of line c at scr[i * L + c]), then copy back
+// scratch of L lines (element i of line c at scr[i * L + c]), then copy back.  The
+// inputs take their twiddles in place first; a thread then sums kBigQ outputs of
+// kBigL lines, so that a value and a root each serve several products.  Each output
+// is the same sum in the same order as one at a time.
+// (The Rayleigh-Ritz step relies on that, so the roundings are spelled out.)  16 FP32
+// spinors of 86^3, the five passes 3.1 -> 2.5 ms; the launch bounds that cap the
+// kernels at 64 registers made every other pass spill.
+template <typename T> constexpr int kBigL = sizeof(T) == 4 ? 4 : 2;
+constexpr int kBigQ = 4;
+__device__ __forceinline__ float2 cmul_rn(float2 a, float2 b)
+{
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ double2 cmul_rn(double2 a, double2 b)
+{
+  return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
 template <typename T>
 __device__ __noinline__ void pass_big(C<T> *buf, int es, int ls, int n, int L, int R, int Ns, const C<T> *__restrict__ tw,
                          bool inv, C<T> *scr)
 {
   const int nb = n / R;
   const int twstep = n / (Ns * R);
-  const int total = n * L;  // one output element per work item
-  for (int wi = threadIdx.x; wi < total; wi += blockDim.x) {
-    const int c = wi % L, rest = wi / L;
-    const int j = rest % nb, q = rest / nb;
-    const int k = j % Ns;
-    const int ob = (j / Ns) * Ns * R + k;
-    const C<T> *x = buf + c * ls;
-    C<T> acc = x[j * es];
-    int e = 0;
-    for (int r = 1; r < R; r++) {
-      e += q;
-      if (e >= R) e -= R;
-      C<T> t1 = tw[r * k * twstep], t2 = tw[e * nb];
-      if (inv) { t1.y = -t1.y; t2.y = -t2.y; }
-      acc = cadd<T>(acc, cmul<T>(cmul<T>(x[(j + r * nb) * es], t1), t2));
+  if (Ns > 1) {
+    for (int wi = threadIdx.x; wi < (n - nb) * L; wi += blockDim.x) {
+      const int c = wi % L, i = nb + wi / L;
+      const int r = i / nb, k = (i - r * nb) % Ns;
+      C<T> t = tw[r * k * twstep];
+      if (inv) t.y = -t.y;
+      C<T> *x = buf + c * ls + i * es;
+      *x = cmul_rn(*x, t);
     }
-    scr[(ob + q * Ns) * L + c] = acc;
+    __syncthreads();
+  }
+  constexpr int NL = kBigL<T>, NQ = kBigQ;
+  const int lg = (L + NL - 1) / NL, qg = (R + NQ - 1) / NQ;
+  for (int wi = threadIdx.x; wi < lg * qg * nb; wi += blockDim.x) {
+    const int c0 = wi % lg, rest = wi / lg;
+    const int j = rest % nb, q0 = (rest / nb) * NQ;
+    const C<T> *x[NL];
+    C<T> acc[NL][NQ];
+#pragma unroll
+    for (int u = 0; u < NL; u++) {
+      x[u] = buf + min(c0 + u * lg, L - 1) * ls + j * es;  // beyond the last line: not stored
+#pragma unroll
+      for (int v = 0; v < NQ; v++) acc[u][v] = *x[u];
+    }
+    int e[NQ];
+#pragma unroll
+    for (int v = 0; v < NQ; v++) e[v] = 0;
+    for (int r = 1; r < R; r++) {
+      C<T> t[NQ];
+#pragma unroll
+      for (int v = 0; v < NQ; v++) {
+        e[v] += q0 + v;
+        if (e[v] >= R) e[v] -= R;
+        if (q0 + v >= R) e[v] = 0;  // beyond the last output: not stored
+        t[v] = tw[e[v] * nb];
+        if (inv) t[v].y = -t[v].y;
+      }
+#pragma unroll
+      for (int u = 0; u < NL; u++) {
+        const C<T> y = x[u][r * nb * es];
+#pragma unroll
+        for (int v = 0; v < NQ; v++) acc[u][v] = cadd<T>(acc[u][v], cmul_rn(y, t[v]));
+      }
+    }
+    const int ob = (j / Ns) * Ns * R + j % Ns;
+#pragma unroll
+    for (int u = 0; u < NL; u++)
+#pragma unroll
+      for (int v = 0; v < NQ; v++)
+        if (c0 + u * lg < L && q0 + v < R) scr[(ob + (q0 + v) * Ns) * L + c0 + u * lg] = acc[u][v];
   }
   __syncthreads();
-  for (int wi = threadIdx.x; wi < total; wi += blockDim.x) {
+  for (int wi = threadIdx.x; wi < n * L; wi += blockDim.x) {
     const int c = wi % L, i = wi / L;
     buf[c * ls + i * es] = scr[i * L + c];
   }
@@ -371,7 +420,7 @@ __global__ void __launch_bounds__(1024, 1) k_fft_plane(const C<T> *__restrict__ 
 // EPI = 1: fused out = a (kin + V phi) + b phi.
 // ---------------------------------------------------------------------------
 template <typename T, int EPI>
-__global__ void __launch_bounds__(256, 4) k_fft_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages st,
+__global__ void __launch_bounds__(256, 2) k_fft_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages st,
                                                const C<T> *__restrict__ twg, long nlines, int L, bool inv,
                                                const C<T> *__restrict__ phi, const T *__restrict__ pot, long ngrid,
                                                T ca, T cb)
@@ -414,7 +463,7 @@ __global__ void __launch_bounds__(256, 4) k_fft_x(const C<T> *__restrict__ in, C
 // KMUL: forward, multiply by the kinetic factor, inverse (z pass only).
 // ---------------------------------------------------------------------------
 template <typename T, bool KMUL>
-__global__ void __launch_bounds__(256, 4) k_fft_cols(C<T> *__restrict__ data, Stages st, const C<T> *__restrict__ twg,
+__global__ void __launch_bounds__(256, 2) k_fft_cols(C<T> *__restrict__ data, Stages st, const C<T> *__restrict__ twg,
                                                   long es, int nxc, int TX, int nxt, long cnt, long s1, long s2,
                                                   bool inv, KinArgs ka)
 {
