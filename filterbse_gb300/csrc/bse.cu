@@ -226,8 +226,7 @@ static int cgemm_nt(fbse_ctx *c, const C<T> *A, int ma, const C<T> *B, int nb, l
 {
   if constexpr (sizeof(T) == 4) {
     if (bse_tensor_cores(c))
-      return tc_complex_nt<float>(c, reinterpret_cast<const float *>(A), ma, reinterpret_cast<const float *>(B), nb,
-                                  L, false, scale, out);
+      return tc_complex_nt(c, A, ma, B, nb, L, scale, out);
   } else {
     // FP64: exact slices on the tensor cores; the SIMT kernel below where the
     // product is short or their scratch does not fit

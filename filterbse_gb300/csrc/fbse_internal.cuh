@@ -306,11 +306,9 @@ int hpsi_fused_apply(fbse_ctx *c, const float2 *in, float2 *out, long nstates, d
 // inverse) in place on nblk FP32 blocks (fft.cu)
 int zpass_kinetic(fbse_ctx *c, float2 *data, long nblk);
 
-// tensor-core complex products (tcgemm.cu):
-//   out[i][j] = scale * sum_r f(A[i][r]) B[j][r], f = conj when conj_a
-template <typename S>
-int tc_complex_nt(fbse_ctx *c, const S *A, int ma, const S *B, int nb, long L, bool conj_a, double scale,
-                  double2 *out);
+// FP32 complex products on the tensor cores (tcgemm.cu):
+//   out[i][j] = scale * sum_r A[i][r] B[j][r]
+int tc_complex_nt(fbse_ctx *c, const float2 *A, int ma, const float2 *B, int nb, long L, double scale, double2 *out);
 
 // FP64 products on the tensor cores by exact integer slices (exactgemm.cu):
 //   out[i][j] = scale * sum_l f(A_i[l]) B_j[l] over L values of each row; rows are
