@@ -66,9 +66,18 @@ static std::vector<int> factorize(int n)
 
 // n = P Q for the two-factor kernels: both radices at most 16 and as close as
 // possible, else the largest P with a register radix up to 31, else with an
-// odd Q up to kSymMax (stage_sym); false: none of them
-constexpr int kSymMin = 27, kSymMax = 255;
-static bool two_factors(int n, int *P, int *Q)
+// odd Q up to kSymMax (stage_sym); false: none of them.
+// Of two radices up to 16 the larger is P on the mixed path's short axes, where the
+// stage that reads global memory has P butterflies a line and too few of them
+// otherwise (2 blocks of 44^3: 23.5 us with 4 x 11, 20.0 with 11 x 4; 57 x 52 x 45:
+// 26.2 and 25.5; 80^3: the same within 2%), and Q on long ones, where more loads in
+// flight per thread pay (8 blocks of 96^3: 123.9 us with 8 x 12, 129.5 with 12 x 8;
+// 116 x 117 x 120: 273 and 281).  FP64 gains from 60 points on with radices up to 10
+// (4 blocks of 60^3 249 -> 244 us, 72^3 451 -> 443, one of 80^3 170 -> 166) and loses
+// below and with larger ones (4 of 45^3 151 -> 159, 8 of 44^3 231 -> 262).
+constexpr int kSymMin = 27, kSymMax = 255, kShortAxis = 80;
+static bool larger_first(int n, int q, bool mixed) { return n <= kShortAxis && (mixed || (n >= 60 && q <= 10)); }
+static bool two_factors(int n, bool mixed, int *P, int *Q)
 {
   for (int set = 0; set < 3; set++)
     for (int p = 16; p >= 1; p--) {
@@ -78,8 +87,9 @@ static bool two_factors(int n, int *P, int *Q)
                           q == 29 || q == 31;
       const bool third = q % 2 == 1 && q >= kSymMin && q <= kSymMax;
       if (set == 0 ? q <= 16 : set == 1 ? second : third) {
-        *P = p;
-        *Q = q;
+        const bool swap = set == 0 && larger_first(n, q, mixed);
+        *P = swap ? q : p;
+        *Q = swap ? p : q;
         return true;
       }
     }
@@ -107,7 +117,7 @@ int plan_axis(fbse_ctx *c, AxisPlan &p, int n)
   FBSE_CUDA(c, cudaMalloc(&p.tw32, n * sizeof(float2)));
   FBSE_CUDA(c, cudaMemcpy(p.tw64, h64.data(), n * sizeof(double2), cudaMemcpyHostToDevice));
   FBSE_CUDA(c, cudaMemcpy(p.tw32, h32.data(), n * sizeof(float2), cudaMemcpyHostToDevice));
-  if (two_factors(n, &p.P, &p.Q)) {
+  if (two_factors(n, c->precision == FBSE_MIXED, &p.P, &p.Q)) {
     std::vector<double2> t64(n);
     std::vector<float2> t32(n);
     for (int k1 = 0; k1 < p.Q; k1++)

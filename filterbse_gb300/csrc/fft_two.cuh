@@ -1,4 +1,4 @@
-// Two-factor FFT kernels for axis lengths n = P Q, P <= Q, P <= 16 a radix that a
+// Two-factor FFT kernels for axis lengths n = P Q, P <= 16 a radix that a
 // thread transforms in registers (fft_radix.cuh) and Q one such radix up to 31,
 // or any odd number of 27 .. 255 (stage_sym): the reference's grid rule gives
 // every even length, so factors 2 x 43 or 4 x 37 are as common as smooth ones.
