@@ -24,8 +24,8 @@
 // round trips and an integer division per element on such lengths, and lengths
 // with a prime above 8 take a direct sum per output.  Measured, H psi through
 // those kernels -> these:
-//   116 x 117 x 120, 4 spinors, FP32 (memory and latency bound)  2101 -> 376 us
-//   96^3, 4 spinors, FP32 (127 terms of a filter)                  742 -> 164 us
+//   116 x 117 x 120, 4 spinors, FP32 (memory and latency bound)  2101 -> 360 us
+//   96^3, 4 spinors, FP32 (127 terms of a filter)                  742 -> 161 us
 //   96^3, 6 spinors, FP64 (FP64 pipe bound; projectors 1.6 ms)     5131 -> 3794 us
 //   57 x 52 x 45, 8 packed states, FP64 (radices 13, 19)           1911 -> 477 us
 #pragma once

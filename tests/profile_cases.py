@@ -12,7 +12,7 @@ the built library.
                                           nCheby 256, 2 nm dot, 32-slot ring (k_newton_acc)
   python tests/profile_cases.py bse       BSE kernel of 16 hole x 16 electron spinor states
                                           of the 2 nm dot, mixed path (k_pair_density,
-                                          convolution FFTs, k_tc_images, k_tc_gemm_nt)
+                                          convolution FFTs, k_tc_gemm_nt)
   python tests/profile_cases.py precond   learned preconditioner on 8 spinor residuals of a
                                           1.6 nm dot, 80^3: inference (k_conv, k_conv16_tc)
                                           and one gradient (k_conv, k_conv_wgrad)
