@@ -46,8 +46,12 @@ struct Stages {
   int n;
   int nst;
   int radix[kMaxStages];
-  int big;  // 1 when a radix exceeds the register limit (needs a scratch line)
+  int big;   // 1 when a radix exceeds the register limit (pass_big)
+  int most;  // butterflies of a line in the register pass that has most
 };
+constexpr int kLineThreads = 256, kPlaneThreads = 1024;
+// the line kernels keep a second set of lines for passes that are not in place
+__host__ __device__ inline bool needs_scratch(const Stages &s) { return s.big || s.most > kLineThreads; }
 
 constexpr int kRegMax = 8;  // odd radices above this take the scratch pass
 
@@ -163,9 +167,12 @@ static Stages stages_of(const AxisPlan &p)
   s.n = p.n;
   s.nst = p.nst;
   s.big = 0;
+  s.most = 0;
   for (int i = 0; i < kMaxStages; i++) {
     s.radix[i] = p.radix[i];
-    if (i < p.nst && p.radix[i] > kRegMax && p.radix[i] != 16) s.big = 1;
+    if (i >= p.nst) continue;
+    if (p.radix[i] > kRegMax && p.radix[i] != 16) s.big = 1;
+    else s.most = std::max(s.most, p.n / p.radix[i]);
   }
   return s;
 }
@@ -204,14 +211,69 @@ __device__ __forceinline__ void dft3(C<T> *v, T sg)
 
 template <typename T, int R> struct IsPow2 { static constexpr bool value = (R & (R - 1)) == 0; };
 
+// a register pass whose lines have more butterflies than the CTA has threads (axes of
+// 514 points and more on the line kernels): in place a thread would have to hold
+// several, so the results go to a scratch of L lines (element i of line c at
+// scr[i * L + c]) and are copied back.  The products of pass_reg.
+template <typename T, int R>
+__device__ __noinline__ void pass_wide(C<T> *buf, int es, int ls, int n, int L, int Ns, const C<T> *__restrict__ tw,
+                                       bool inv, C<T> *scr)
+{
+  const int nb = n / R, twstep = n / (Ns * R);
+  const T sg = inv ? T(1) : T(-1);
+  for (int wi = threadIdx.x; wi < nb * L; wi += blockDim.x) {
+    const int c = wi % L, j = wi / L, k = j % Ns;
+    const C<T> *x = buf + c * ls;
+    C<T> v[R];
+    v[0] = x[j * es];
+#pragma unroll
+    for (int q = 1; q < R; q++) {
+      C<T> t = tw[q * k * twstep];
+      if (inv) t.y = -t.y;
+      v[q] = cmul<T>(x[(j + q * nb) * es], t);
+    }
+    C<T> *o = scr + ((j / Ns) * Ns * R + k) * L + c;
+    if constexpr (IsPow2<T, R>::value) {
+      dif_pow2<T, R>(v, sg);
+#pragma unroll
+      for (int q = 0; q < R; q++) o[q * Ns * L] = v[bitrev(q, ilog2(R))];
+    } else {
+      if constexpr (R == 3) {
+        dft3<T>(v, sg);
+      } else {
+        C<T> w[R];
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+          w[e] = tw[e * nb];
+          if (inv) w[e].y = -w[e].y;
+        }
+        dft_odd<T, R>(v, w);
+      }
+#pragma unroll
+      for (int q = 0; q < R; q++) o[q * Ns * L] = v[q];
+    }
+  }
+  __syncthreads();
+  for (int wi = threadIdx.x; wi < n * L; wi += blockDim.x) {
+    const int c = wi % L, i = wi / L;
+    buf[c * ls + i * es] = scr[i * L + c];
+  }
+  __syncthreads();
+}
+
 // ---------------------------------------------------------------------------
 // one in-place Stockham pass of radix R over L lines (element i of line c at
-// buf[c * ls + i * es]); lanes take consecutive lines at one butterfly index
+// buf[c * ls + i * es]); lanes take consecutive lines at one butterfly index.
+// scr: needed where a line has more butterflies than the CTA threads (pass_wide)
 // ---------------------------------------------------------------------------
 template <typename T, int R>
 __device__ __forceinline__ void pass_reg(C<T> *buf, int es, int ls, int n, int L, int Ns, const C<T> *__restrict__ tw,
-                                      bool inv)
+                                      bool inv, C<T> *scr)
 {
+  if (n / R > (int)blockDim.x) {
+    pass_wide<T, R>(buf, es, ls, n, L, Ns, tw, inv, scr);
+    return;
+  }
   constexpr int kMaxE = R;                              // one butterfly per thread per round
   constexpr int BMAX = (kMaxE / R) > 0 ? kMaxE / R : 1;
   const int nb = n / R;
@@ -362,13 +424,13 @@ __device__ void fft_lines(C<T> *buf, int es, int ls, int L, const Stages &st, co
   for (int s = 0; s < st.nst; s++) {
     const int R = st.radix[s];
     switch (R) {
-      case 2: pass_reg<T, 2>(buf, es, ls, st.n, L, Ns, tw, inv); break;
-      case 3: pass_reg<T, 3>(buf, es, ls, st.n, L, Ns, tw, inv); break;
-      case 4: pass_reg<T, 4>(buf, es, ls, st.n, L, Ns, tw, inv); break;
-      case 5: pass_reg<T, 5>(buf, es, ls, st.n, L, Ns, tw, inv); break;
-      case 7: pass_reg<T, 7>(buf, es, ls, st.n, L, Ns, tw, inv); break;
-      case 8: pass_reg<T, 8>(buf, es, ls, st.n, L, Ns, tw, inv); break;
-      case 16: pass_reg<T, 16>(buf, es, ls, st.n, L, Ns, tw, inv); break;
+      case 2: pass_reg<T, 2>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 3: pass_reg<T, 3>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 4: pass_reg<T, 4>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 5: pass_reg<T, 5>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 7: pass_reg<T, 7>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 8: pass_reg<T, 8>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 16: pass_reg<T, 16>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
       default: pass_big<T>(buf, es, ls, st.n, L, R, Ns, tw, inv, scr); break;
     }
     Ns *= R;
@@ -382,7 +444,7 @@ __device__ void fft_lines(C<T> *buf, int es, int ls, int L, const Stages &st, co
 //   MODE 1: inverse y then x, epilogue out = a (kin + V phi) + b phi
 // ---------------------------------------------------------------------------
 template <typename T, int MODE>
-__global__ void __launch_bounds__(1024, 1) k_fft_plane(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages sx,
+__global__ void __launch_bounds__(kPlaneThreads, 1) k_fft_plane(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages sx,
                                                    Stages sy, const C<T> *__restrict__ twxg,
                                                    const C<T> *__restrict__ twyg, const C<T> *__restrict__ phi,
                                                    const T *__restrict__ pot, long ngrid, T ca, T cb)
@@ -430,7 +492,7 @@ __global__ void __launch_bounds__(1024, 1) k_fft_plane(const C<T> *__restrict__ 
 // EPI = 1: fused out = a (kin + V phi) + b phi.
 // ---------------------------------------------------------------------------
 template <typename T, int EPI>
-__global__ void __launch_bounds__(256, 2) k_fft_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages st,
+__global__ void __launch_bounds__(kLineThreads, 2) k_fft_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages st,
                                                const C<T> *__restrict__ twg, long nlines, int L, bool inv,
                                                const C<T> *__restrict__ phi, const T *__restrict__ pot, long ngrid,
                                                T ca, T cb)
@@ -439,7 +501,7 @@ __global__ void __launch_bounds__(256, 2) k_fft_x(const C<T> *__restrict__ in, C
   const int n = st.n, np = n | 1;
   C<T> *tw = reinterpret_cast<C<T> *>(smem_raw);
   C<T> *A = tw + n;
-  C<T> *S = A + (long)L * np;  // scratch for a radix above the register limit
+  C<T> *S = A + (long)L * np;  // scratch (needs_scratch)
   for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];
   const long line0 = (long)blockIdx.x * L;
   const int nl = (int)min((long)L, nlines - line0);
@@ -447,7 +509,7 @@ __global__ void __launch_bounds__(256, 2) k_fft_x(const C<T> *__restrict__ in, C
 #pragma unroll 8
   for (int t = threadIdx.x; t < nl * n; t += blockDim.x) A[(t / n) * np + t % n] = in[off + t];
   __syncthreads();
-  fft_lines<T>(A, 1, np, nl, st, tw, inv, st.big ? S : nullptr);
+  fft_lines<T>(A, 1, np, nl, st, tw, inv, needs_scratch(st) ? S : nullptr);
 #pragma unroll 8
   for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
     C<T> v = A[(t / n) * np + t % n];
@@ -473,7 +535,7 @@ __global__ void __launch_bounds__(256, 2) k_fft_x(const C<T> *__restrict__ in, C
 // KMUL: forward, multiply by the kinetic factor, inverse (z pass only).
 // ---------------------------------------------------------------------------
 template <typename T, bool KMUL>
-__global__ void __launch_bounds__(256, 2) k_fft_cols(C<T> *__restrict__ data, Stages st, const C<T> *__restrict__ twg,
+__global__ void __launch_bounds__(kLineThreads, 2) k_fft_cols(C<T> *__restrict__ data, Stages st, const C<T> *__restrict__ twg,
                                                   long es, int nxc, int TX, int nxt, long cnt, long s1, long s2,
                                                   bool inv, KinArgs ka)
 {
@@ -481,7 +543,7 @@ __global__ void __launch_bounds__(256, 2) k_fft_cols(C<T> *__restrict__ data, St
   const int n = st.n;
   C<T> *tw = reinterpret_cast<C<T> *>(smem_raw);
   C<T> *A = tw + n;
-  C<T> *S = A + (long)TX * n;  // scratch for a radix above the register limit
+  C<T> *S = A + (long)TX * n;  // scratch (needs_scratch)
   for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];
   const long o = blockIdx.x / nxt;
   const int xt = blockIdx.x % nxt;
@@ -494,7 +556,7 @@ __global__ void __launch_bounds__(256, 2) k_fft_cols(C<T> *__restrict__ data, St
     A[i * L + cc] = data[base + (long)i * es + cc];
   }
   __syncthreads();
-  fft_lines<T>(A, L, 1, L, st, tw, KMUL ? false : inv, st.big ? S : nullptr);
+  fft_lines<T>(A, L, 1, L, st, tw, KMUL ? false : inv, needs_scratch(st) ? S : nullptr);
   if (KMUL) {
     const int jy = (int)(o % cnt);
     if (ka.kq) {
@@ -511,7 +573,7 @@ __global__ void __launch_bounds__(256, 2) k_fft_cols(C<T> *__restrict__ data, St
       }
     }
     __syncthreads();
-    fft_lines<T>(A, L, 1, L, st, tw, true, st.big ? S : nullptr);
+    fft_lines<T>(A, L, 1, L, st, tw, true, needs_scratch(st) ? S : nullptr);
   }
 #pragma unroll 8
   for (int t = threadIdx.x; t < n * L; t += blockDim.x) {
@@ -556,15 +618,15 @@ static int launch_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv,
   const long nlines = nblk * c->ny * c->nz;
   Stages st = stages_of(p);
   int L = 32;
-  while (L > 1 && (size_t)(n + (st.big ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>) > (size_t)max_smem()) L /= 2;
-  const size_t smem = (size_t)(n + (st.big ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>);
+  while (L > 1 && (size_t)(n + (needs_scratch(st) ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>) > (size_t)max_smem()) L /= 2;
+  const size_t smem = (size_t)(n + (needs_scratch(st) ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>);
   const long grid = (nlines + L - 1) / L;
   if (epi) {
     FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_x<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_x<T, 1><<<grid, 256, smem, c->stream>>>(in, out, st, roots<T>(p), nlines, L, inv, phi, pot, c->ngrid, ca, cb);
+    k_fft_x<T, 1><<<grid, kLineThreads, smem, c->stream>>>(in, out, st, roots<T>(p), nlines, L, inv, phi, pot, c->ngrid, ca, cb);
   } else {
     FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_x<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_x<T, 0><<<grid, 256, smem, c->stream>>>(in, out, st, roots<T>(p), nlines, L, inv, nullptr, nullptr,
+    k_fft_x<T, 0><<<grid, kLineThreads, smem, c->stream>>>(in, out, st, roots<T>(p), nlines, L, inv, nullptr, nullptr,
                                                    c->ngrid, T(1), T(0));
   }
   FBSE_CHECK_LAUNCH(c);
@@ -585,7 +647,11 @@ static int launch_cols(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, b
 {
   const AxisPlan &p = c->ax[axis];
   const int n = p.n;
-  const int TX = cols_tile((int)c->nx, (int)sizeof(C<T>));
+  const Stages st = stages_of(p);
+  int TX = cols_tile((int)c->nx, (int)sizeof(C<T>));
+  auto bytes = [&] { return (size_t)(n + (needs_scratch(st) ? 2L : 1L) * TX * n) * sizeof(C<T>); };
+  // narrower tiles where a long axis' register passes need the scratch
+  while (!st.big && needs_scratch(st) && TX > 1 && bytes() > (size_t)max_smem()) TX = (TX + 1) / 2;
   const int nxt = (int)((c->nx + TX - 1) / TX);
   long es, cnt, s1, s2, nouter;
   if (axis == 1) {  // y lines: outer = block*nz + z
@@ -601,17 +667,16 @@ static int launch_cols(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, b
     s2 = c->nx;
     nouter = nblk * c->ny;
   }
-  Stages st = stages_of(p);
-  const size_t smem = (size_t)(n + (st.big ? 2L : 1L) * TX * n) * sizeof(C<T>);
+  const size_t smem = bytes();
   if (smem > (size_t)max_smem()) return set_err(c, FBSE_ERR_UNSUPPORTED, "FFT axis too long for shared memory");
   const long grid = nouter * nxt;
   if (kmul) {
     FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_cols<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_cols<T, true><<<grid, 256, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1, s2,
+    k_fft_cols<T, true><<<grid, kLineThreads, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1, s2,
                                                          inv, ka);
   } else {
     FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_cols<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_cols<T, false><<<grid, 256, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1,
+    k_fft_cols<T, false><<<grid, kLineThreads, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1,
                                                           s2, inv, ka);
   }
   FBSE_CHECK_LAUNCH(c);
@@ -633,11 +698,11 @@ static int launch_plane(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, int m
   Stages sx = stages_of(c->ax[0]), sy = stages_of(c->ax[1]);
   if (mode == 0) {
     FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_plane<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_plane<T, 0><<<grid, 1024, smem, c->stream>>>(in, out, sx, sy, roots<T>(c->ax[0]), roots<T>(c->ax[1]),
+    k_fft_plane<T, 0><<<grid, kPlaneThreads, smem, c->stream>>>(in, out, sx, sy, roots<T>(c->ax[0]), roots<T>(c->ax[1]),
                                                        nullptr, nullptr, c->ngrid, T(1), T(0));
   } else {
     FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_plane<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_plane<T, 1><<<grid, 1024, smem, c->stream>>>(in, out, sx, sy, roots<T>(c->ax[0]), roots<T>(c->ax[1]), phi,
+    k_fft_plane<T, 1><<<grid, kPlaneThreads, smem, c->stream>>>(in, out, sx, sy, roots<T>(c->ax[0]), roots<T>(c->ax[1]), phi,
                                                        pot, c->ngrid, ca, cb);
   }
   FBSE_CHECK_LAUNCH(c);
@@ -832,7 +897,8 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
   // memory, or y and x lines with the same arithmetic in the same order
   const bool both = !fplane && c->tune.fft_kernels == 0 && !c->steady && c->ax[0].P > 0 && c->ax[1].P > 0;
   const bool lines = two_axis_ok(c, 0) || two_axis_ok(c, 1);
-  const bool plane = !lines && !sx.big && !sy.big && plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;
+  const bool plane = !lines && !sx.big && !sy.big && std::max(sx.most, sy.most) <= kPlaneThreads &&
+                     plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;
   // which of x and y the z pass meets in a two-factor transform's order
   const bool xo = both || (!fplane && !plane && two_axis_ok(c, 0));
   const bool yo = both || (!fplane && !plane && two_axis_ok(c, 1));
