@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char *stage = smem_raw + ((128 - (smem_u32(smem_raw) & 127)) & 127);
-  __shared__ __align__(8) uint64_t full_bar[2], free_bar[2], sums_bar, read_bar;
+  __shared__ __align__(8) uint64_t full_bar[2], free_bar[2], sums_bar, read_bar, last_bar;
   __shared__ uint32_t tmem_base;
   __shared__ int fail;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&free_bar[s], 1);
     }
     mbar_init(&sums_bar, 1);
+    mbar_init(&last_bar, 1);
     mbar_init(&read_bar, kReadWarps);
     fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -117,8 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base;
-  int issued = 0;      // stages copied (thread 0)
-  int committed = 0;   // read-outs handed over (thread 32)
+  int issued = 0;  // stages copied (thread 0)
   if (threadIdx.x == 0) {
     const unsigned char *a = A + ((long)blockIdx.x * nkb + kb0) * kStageA;
     const unsigned char *b = B + ((long)blockIdx.y * nkb + kb0) * kStageB;
@@ -155,11 +155,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 i == 0 ? first : 1u);
       }
       commit(&free_bar[s]);
-      if (it % kDrain == kDrain - 1 || it == nk - 1) {
-        commit(&sums_bar);
-        committed++;
-      }
+      if (it % kDrain == kDrain - 1 || it == nk - 1) commit(&sums_bar);
     }
+    commit(&last_bar);  // arrives once every MMA issued is done, whichever wait ended the loop
     if (!ok) atomicExch(&fail, 1);
   } else if (warp >= 2) {
     // lanes: rows 32 (warp % 4) ..; columns: half of the tile
@@ -220,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       atomicExch(status, 1);
       for (int it = issued > 2 ? issued - 2 : 0; it < issued; it++) mbar_wait(&full_bar[it & 1], (uint32_t)((it >> 1) & 1));
     }
-    if (threadIdx.x == 32 && committed > 0) mbar_wait(&sums_bar, (uint32_t)((committed - 1) & 1));
+    if (threadIdx.x == 32) mbar_wait(&last_bar, 0u);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
