@@ -47,6 +47,11 @@ constexpr int kSlices = 8, kOrders = 8;
 constexpr int kTileA = kM * kK * 2, kTileB = kN * kK * 2;  // bytes of one slice
 constexpr int kStageA = kSlices * kTileA, kStageB = kSlices * kTileB, kStage = kStageA + kStageB;
 constexpr int kDrain = 128 / kK;        // stages between read-outs
+// stages per split.  Fixed, and chunks of K are whole splits added in order, so a
+// result's bits depend on the rows' length alone: not on how many rows there are, nor
+// on the room for the images.  64: a CTA's start and end cost six stages, and the 16
+// tiles of 196 x 196 complex products of 85184 points fill 8.8 waves of 152 CTAs.
+constexpr int kSplit = 64;
 constexpr int kReadWarps = 8, kThreads = 32 * (2 + kReadWarps);
 constexpr int kCols = kN / 2;           // columns of a reading thread
 constexpr int kNonFinite = 1 << 20;     // exponent of a row that holds an infinity or NaN
@@ -86,7 +91,7 @@ __device__ __forceinline__ void arrive(uint64_t *bar)
 // ea [split][mp], eb [split][n1]: the rows' exponents (n1 = np, or np / 2 when B's
 // second half of rows rearranges the first).
 __global__ void __launch_bounds__(kThreads, 1)
-    k_ex_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__ B, long nkb, long kb_per_split,
+    k_ex_gemm(const unsigned char *__restrict__ A, const unsigned char *__restrict__ B, long nkb,
               const int *__restrict__ ea, const int *__restrict__ eb, double *__restrict__ part, long mp, long np,
               long n1, int *__restrict__ status)
 {
@@ -96,8 +101,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ uint32_t tmem_base;
   __shared__ int fail;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long kb0 = (long)blockIdx.z * kb_per_split;
-  const int nk = (int)(min(nkb, kb0 + kb_per_split) - kb0);
+  const long kb0 = (long)blockIdx.z * kSplit;
+  const int nk = (int)(min(nkb, kb0 + kSplit) - kb0);
   const int ndrain = (nk + kDrain - 1) / kDrain;
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; s++) {
@@ -227,12 +232,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // exponent of each (row, split): 2^e above twice the largest magnitude
 __global__ void __launch_bounds__(256) k_ex_exp(const double *__restrict__ src, long ld, int nrows, long k_len, long k0,
-                                                long k_split, long rows_p, int *__restrict__ e)
+                                                long rows_p, int *__restrict__ e)
 {
   const long row = blockIdx.x;
   int ex = -1021;
   if (row < nrows) {
-    const long b = k0 + blockIdx.y * k_split, end = min(k_len, b + k_split);
+    const long b = k0 + (long)blockIdx.y * kSplit * kK, end = min(k_len, b + kSplit * kK);
     unsigned m = 0;  // biased exponents
     for (long k = b + threadIdx.x; k < end; k += blockDim.x)
       m = max(m, ((unsigned)__double2hiint(src[row * ld + k]) >> 20) & 0x7ffu);
@@ -252,8 +257,8 @@ __global__ void __launch_bounds__(256) k_ex_exp(const double *__restrict__ src, 
 //   0: x[k]   1: odd k negated   2: pairs swapped   3: pairs swapped, odd k negated
 template <int ROWS>
 __global__ void __launch_bounds__(256)
-    k_ex_slice(const double *__restrict__ src, long ld, int nrows, long k_len, long k0, long kb_per_split, int mode,
-               long rows_p, long nkb, const int *__restrict__ e, unsigned char *__restrict__ img)
+    k_ex_slice(const double *__restrict__ src, long ld, int nrows, long k_len, long k0, int mode, long rows_p, long nkb,
+               const int *__restrict__ e, unsigned char *__restrict__ img)
 {
   constexpr int kTile = ROWS * kK * 2;
   const long total = rows_p * nkb * 4;
@@ -261,7 +266,7 @@ __global__ void __launch_bounds__(256)
     const long row = t % rows_p, kc = t / rows_p, kb = kc / 4;
     const int c16 = (int)(kc % 4);
     const long k = k0 + kc * 8;
-    const int ea = e[(kb / kb_per_split) * rows_p + row];
+    const int ea = e[(kb / kSplit) * rows_p + row];
     uint32_t word[kSlices][4];
     unsigned long long prev = 0;
 #pragma unroll
@@ -297,43 +302,26 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// out[i][j] (+)= scale * (sum of the splits' real columns, imaginary columns)
+// out[i][j] = scale * (sum of the splits' real columns, imaginary columns), the splits
+// of all chunks in order: a chunk adds to the sums of those before it, the last one scales
 __global__ void k_ex_reduce(const double *__restrict__ part, int nsplit, long mp, long np, int m, int n, long im_col,
-                            double scale, int add, double2 *__restrict__ out)
+                            bool first, bool last, double scale, double2 *__restrict__ out)
 {
   const long total = (long)m * n;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
     const long i = e / n, j = e % n;
-    double re = 0, im = 0;
+    double2 o = first ? make_double2(0, 0) : out[e];
+#pragma unroll 4
     for (int s = 0; s < nsplit; s++) {
       const double *p = part + ((long)s * mp + i) * np;
-      re += p[j];
-      if (im_col) im += p[im_col + j];
+      o.x += p[j];
+      if (im_col) o.y += p[im_col + j];
     }
-    const double2 o = add ? out[e] : make_double2(0, 0);
-    out[e] = make_double2(o.x + re * scale, o.y + im * scale);
+    out[e] = last ? make_double2(o.x * scale, o.y * scale) : o;
   }
 }
 
 }  // namespace ex
-
-// splits of the K blocks of one chunk: whole waves of 152 CTAs, at most 1024 blocks
-// (one exponent for 32768 values)
-static long ex_splits(long tiles, long nkb)
-{
-  const long least = (nkb + 1023) / 1024;
-  long best = least;
-  double cost = 1e300;
-  for (long s = least; s <= std::max<long>(least, std::min<long>(nkb, 2 * least + 152)); s++) {
-    const double waves = (double)((tiles * s + 151) / 152);
-    const double t = waves * ((double)((nkb + s - 1) / s) + 6.0);  // a CTA's start and end: about six stages
-    if (t < cost) {
-      cost = t;
-      best = s;
-    }
-  }
-  return best;
-}
 
 int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, long ldb, int nb, long L, ExactKind kind,
              double scale, double2 *out)
@@ -345,15 +333,13 @@ int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, lo
   const long K = cplx ? 2 * L : L;
   const long mp = (ma + kM - 1) / kM * kM, n1 = (nb + kN - 1) / kN * kN, np = cplx ? 2 * n1 : n1;
   const long nkb_all = (K + kK - 1) / kK;
-  // images of a K chunk within 4 GB, its partial sums within 2 GB
+  // images of a K chunk within 4 GB (fbse_tuning.tc_image_bytes sets another size), its
+  // partial sums within 2 GB, at least one split
   const long row_bytes = (long)kSlices * kK * 2;
-  long nkb = std::min<long>(nkb_all, std::max<long>(1, 4000000000L / (row_bytes * (mp + np))));
-  nkb = std::min<long>(nkb, 1024 * std::max<long>(1, 2000000000L / (8 * mp * np)));
-  const long nchunk = (nkb_all + nkb - 1) / nkb;
-  nkb = (nkb_all + nchunk - 1) / nchunk;
-  const long tiles = (mp / kM) * (np / kN);
-  const long want = ex_splits(tiles, nkb);
-  const long kbs = (nkb + want - 1) / want, nsplit = (nkb + kbs - 1) / kbs;
+  const double budget = c->tune.tc_image_bytes > 0 ? c->tune.tc_image_bytes : 4.0e9;
+  const long fit = std::min((long)(budget / (double)(row_bytes * (mp + np))) / kSplit, 2000000000L / (8 * mp * np));
+  const long nsplit_all = (nkb_all + kSplit - 1) / kSplit, nchunk = (nsplit_all + std::max(1L, fit) - 1) / std::max(1L, fit);
+  const long nsplit = (nsplit_all + nchunk - 1) / nchunk, nkb = std::min(nkb_all, nsplit * kSplit);
   const size_t img_a = (size_t)(mp * nkb * row_bytes), img_b = (size_t)(np * nkb * row_bytes);
   const size_t part_b = (size_t)nsplit * mp * np * sizeof(double), exp_b = (size_t)nsplit * (mp + n1) * sizeof(int);
   void *scratch = nullptr;
@@ -368,24 +354,24 @@ int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, lo
   const int mode_b[2] = {kind == kExactPlain ? 1 : 0, kind == kExactPlain ? 2 : 3};
   auto grid = [](long n) { return (unsigned)std::min<long>((n + 255) / 256, 152 * 32); };
   for (long ch = 0; ch < nchunk; ch++) {
-    const long k0 = ch * nkb * kK, kb = std::min<long>(nkb, nkb_all - ch * nkb);
-    const long ns = (kb + kbs - 1) / kbs;
-    k_ex_exp<<<dim3((unsigned)mp, (unsigned)ns), 256, 0, c->stream>>>(A, lda, ma, K, k0, kbs * kK, mp, ea);
+    const long kb0 = ch * nsplit * kSplit, kb = std::min(nkb, nkb_all - kb0), k0 = kb0 * kK;
+    const long ns = (kb + kSplit - 1) / kSplit;
+    k_ex_exp<<<dim3((unsigned)mp, (unsigned)ns), 256, 0, c->stream>>>(A, lda, ma, K, k0, mp, ea);
     FBSE_CHECK_LAUNCH(c);
-    k_ex_slice<kM><<<grid(mp * kb * 4), 256, 0, c->stream>>>(A, lda, ma, K, k0, kbs, 0, mp, kb, ea, ia);
+    k_ex_slice<kM><<<grid(mp * kb * 4), 256, 0, c->stream>>>(A, lda, ma, K, k0, 0, mp, kb, ea, ia);
     FBSE_CHECK_LAUNCH(c);
-    k_ex_exp<<<dim3((unsigned)n1, (unsigned)ns), 256, 0, c->stream>>>(B, ldb, nb, K, k0, kbs * kK, n1, eb);
+    k_ex_exp<<<dim3((unsigned)n1, (unsigned)ns), 256, 0, c->stream>>>(B, ldb, nb, K, k0, n1, eb);
     FBSE_CHECK_LAUNCH(c);
     for (int h = 0; h < (cplx ? 2 : 1); h++) {
-      k_ex_slice<kN><<<grid(n1 * kb * 4), 256, 0, c->stream>>>(B, ldb, nb, K, k0, kbs, mode_b[h], n1, kb, eb,
+      k_ex_slice<kN><<<grid(n1 * kb * 4), 256, 0, c->stream>>>(B, ldb, nb, K, k0, mode_b[h], n1, kb, eb,
                                                                ib + (size_t)h * n1 * kb * row_bytes);
       FBSE_CHECK_LAUNCH(c);
     }
     k_ex_gemm<<<dim3((unsigned)(mp / kM), (unsigned)(np / kN), (unsigned)ns), kThreads, kSmem, c->stream>>>(
-        ia, ib, kb, kbs, ea, eb, part, mp, np, n1, status);
+        ia, ib, kb, ea, eb, part, mp, np, n1, status);
     FBSE_CHECK_LAUNCH(c);
-    k_ex_reduce<<<grid((long)ma * nb), 256, 0, c->stream>>>(part, (int)ns, mp, np, ma, nb, cplx ? n1 : 0, scale, ch > 0,
-                                                             out);
+    k_ex_reduce<<<grid((long)ma * nb), 256, 0, c->stream>>>(part, (int)ns, mp, np, ma, nb, cplx ? n1 : 0, ch == 0,
+                                                             ch == nchunk - 1, scale, out);
     FBSE_CHECK_LAUNCH(c);
   }
   int hs = 0;

@@ -127,7 +127,9 @@ typedef struct fbse_tuning {
   int newton_ring;         /* Newton ring slots, 8..128 (the FP32 block sums depend on it); 0: 128 */
   int bse_simt;            /* 1: the mixed path's BSE contraction on the FP32 SIMT kernel instead of
                               the tensor cores */
-  double tc_image_bytes;   /* split operands of the mixed path's BSE contraction one launch covers, bytes; 0: 24e9 */
+  double tc_image_bytes;   /* operands one launch of a tensor-core product covers, bytes: the split rows of the
+                              mixed path's BSE contraction (0: 24e9), the slices of FP64 products (0: 4e9).  FP64
+                              results do not depend on it */
   double ritz_cut;         /* overlap eigenvalues kept by fbse_ortho_diag_sigma, relative to the largest
                               (the role of SVDEPS, filter_mpi/fd.h); 0: 1e-12 (FP64), the mixed path's own
                               default otherwise */
