@@ -257,7 +257,10 @@ int fbse_angular_stats(fbse_ctx *ctx, const double *psitot, long n, const double
  * the slab Grams is the Gram of the whole states, and each process rotates its
  * own slab.
  *   fbse_gram:   out[i][j] = dv sum_l conj(A_i[l]) B_j[l], na x nb complex
- *                (host, row-major, (re, im) pairs); A, B device psitot rows.
+ *                (host, row-major, (re, im) pairs); A, B device psitot rows.  Each
+ *                element is as accurate as an FP64 sum, relative to dv sum |A_i||B_j|;
+ *                from 2048 values on, those of a row that holds an infinity or a
+ *                NaN are NaN.
  *   fbse_rotate: out_j[l] = sum_i coef[i][j] A_i[l] for j < k, l in the slab;
  *                coef host na x k complex, row-major; out device psitot rows
  *                (values outside the slab untouched), not aliasing A. */
