@@ -150,11 +150,11 @@ extern "C" int fbse_angular_stats(fbse_ctx *c, const double *psitot, long n, con
   double *dk = nullptr, *dg = nullptr, *part = nullptr;
   const long naxes = c->nx + c->ny + c->nz;
   int rc = FBSE_OK;
-  if (cudaMalloc(&kq, 4 * N * sizeof(double2)) != cudaSuccess || cudaMalloc(&lp, nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&P, 3 * nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&work, nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&dk, naxes * sizeof(double)) != cudaSuccess || cudaMalloc(&dg, naxes * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&part, (size_t)kAngBlocks * 8 * sizeof(double)) != cudaSuccess) {
+  if (dev_alloc(c, &kq, 4 * N * sizeof(double2)) != cudaSuccess || dev_alloc(c, &lp, nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &P, 3 * nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &work, nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &dk, naxes * sizeof(double)) != cudaSuccess || dev_alloc(c, &dg, naxes * sizeof(double)) != cudaSuccess ||
+      dev_alloc(c, &part, (size_t)kAngBlocks * 8 * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     rc = set_err(c, FBSE_ERR_OOM, "fbse_angular_stats");
   }

@@ -37,7 +37,7 @@ int ensure(fbse_ctx *c, void **p, size_t *have, size_t need)
     *have = 0;
   }
   if (need == 0) return FBSE_OK;
-  if (cudaMalloc(p, need) != cudaSuccess) {
+  if (dev_alloc(c, p, need) != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
     return set_err(c, FBSE_ERR_OOM, "device allocation of " + std::to_string(need) + " bytes failed");
@@ -73,7 +73,7 @@ template <typename D, typename S> static int upload(fbse_ctx *c, D **dst, const 
 {
   std::vector<D> tmp(n);
   for (size_t i = 0; i < n; i++) tmp[i] = (D)src[i];
-  FBSE_CUDA(c, cudaMalloc(dst, n * sizeof(D) + 16));
+  FBSE_CUDA(c, dev_alloc(c, dst, n * sizeof(D) + 16));
   FBSE_CUDA(c, cudaMemcpy(*dst, tmp.data(), n * sizeof(D), cudaMemcpyHostToDevice));
   return FBSE_OK;
 }
@@ -403,7 +403,7 @@ static int create(fbse_ctx *c, const fbse_grid_desc *g, const double *pot, const
       if ((rc = upload(c, &p.pe_nlpf, pn.data(), pn.size()))) return rc;
       if ((rc = build_plane_table(c, cj, cb, pa, py, ps, pn, nent))) return rc;
     }
-    FBSE_CUDA(c, cudaMalloc(&p.LS, 36 * sizeof(double2)));
+    FBSE_CUDA(c, dev_alloc(c, &p.LS, 36 * sizeof(double2)));
     FBSE_CUDA(c, cudaMemcpy(p.LS, ls, 36 * sizeof(double2), cudaMemcpyHostToDevice));
   }
   return FBSE_OK;
@@ -472,7 +472,7 @@ void fbse_destroy(fbse_ctx *c)
 int fbse_alloc(fbse_ctx *c, void **dptr, size_t bytes)
 {
   if (!c || !dptr) return FBSE_ERR_ARG;
-  if (cudaMalloc(dptr, bytes ? bytes : 1) != cudaSuccess) {
+  if (dev_alloc(c, dptr, bytes ? bytes : 1) != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, FBSE_ERR_OOM, "fbse_alloc of " + std::to_string(bytes) + " bytes failed");
   }

@@ -80,7 +80,7 @@ int fbse_batch_create(fbse_batch **out, const fbse_batch_dot *dots, int ndots)
     b->zn.emplace_back(d.zn, d.zn + d.ncheby);
     b->an.emplace_back(d.an, d.an + 2 * d.m * d.ncheby);
     double *a = nullptr;
-    if (cudaMalloc(&a, (size_t)d.m * d.ncheby * sizeof(double)) != cudaSuccess) {
+    if (dev_alloc(d.ctx, &a, (size_t)d.m * d.ncheby * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
       rc = berr(b, FBSE_ERR_OOM, "dot " + std::to_string(i) + ": coefficients");
       break;

@@ -241,7 +241,7 @@ static int cgemm_nt(fbse_ctx *c, const C<T> *A, int ma, const C<T> *B, int nb, l
   while (nchunk > 1 && (double)nchunk * ma * nb * 16.0 > 8.0e9) nchunk /= 2;
   const long kchunk = (L + nchunk - 1) / nchunk;
   double2 *part = nullptr;
-  if (cudaMalloc(&part, (size_t)nchunk * ma * nb * sizeof(double2)) != cudaSuccess) {
+  if (dev_alloc(c, &part, (size_t)nchunk * ma * nb * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, FBSE_ERR_OOM, "bse gemm partials");
   }
@@ -340,12 +340,7 @@ static int eh_kernels_t(fbse_ctx *c, const double *psi_qp, long nh, long ne, lon
   double2 *G = nullptr;
   const long maxrows = std::max(ne * ne, std::max(nh * nh, nx));
   auto fail = [&](const char *m) { cudaGetLastError(); rc = set_err(c, FBSE_ERR_OOM, m); };
-  auto get = [&](auto **p, size_t bytes) {
-    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
-    cudaGetLastError();
-    release(c, kSlotTc);  // an earlier product's scratch
-    return cudaMalloc(p, bytes) == cudaSuccess;
-  };
+  auto get = [&](auto **p, size_t bytes) { return dev_alloc(c, p, bytes) == cudaSuccess; };
   if (!get(&P, (size_t)maxrows * N * sizeof(C<T>))) fail("bse pair densities");
   else if (!get(&Q, (size_t)maxrows * N * sizeof(C<T>))) fail("bse pair densities");
   else if (!get(&wk, (size_t)2 * batch * N * sizeof(C<T>))) fail("bse fft scratch");
@@ -725,8 +720,8 @@ int fbse_bse_potentials(fbse_ctx *c, const double *gx, const double *gy, const d
   double *dg = nullptr;
   double2 *work = nullptr;
   int rc = FBSE_OK;
-  if (cudaMalloc(&dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&work, (size_t)N * sizeof(double2)) != cudaSuccess) {
+  if (dev_alloc(c, &dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess ||
+      dev_alloc(c, &work, (size_t)N * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
     if (dg) cudaFree(dg);
     return set_err(c, FBSE_ERR_OOM, "fbse_bse_potentials");
@@ -776,8 +771,8 @@ int fbse_bse_kernel_real(fbse_ctx *c, const double *psi_qp, long n_h, long n_e, 
   if (c->nspin != 1) return set_err(c, FBSE_ERR_UNSUPPORTED, "fbse_bse_kernel_real: one spin component per state");
   const long N = c->ngrid, nq = lumo_idx + n_e, nx = n_h * n_e;
   double2 *pc = nullptr, *dc = nullptr, *xc = nullptr;
-  if (cudaMalloc(&pc, nq * N * sizeof(double2)) != cudaSuccess || cudaMalloc(&dc, nx * nx * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&xc, nx * nx * sizeof(double2)) != cudaSuccess) {
+  if (dev_alloc(c, &pc, nq * N * sizeof(double2)) != cudaSuccess || dev_alloc(c, &dc, nx * nx * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &xc, nx * nx * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
     if (pc) cudaFree(pc);
     if (dc) cudaFree(dc);
@@ -822,9 +817,9 @@ int fbse_bse_solve(fbse_ctx *c, const double *eval_qp_host, long n_qp, long n_h,
   double2 *H = nullptr, *V = nullptr, *T1 = nullptr, *Cm = nullptr;
   int *perm_d = nullptr;
   int rc = FBSE_OK;
-  if (cudaMalloc(&ev, n_qp * sizeof(double)) != cudaSuccess || cudaMalloc(&dots, 4 * n * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&H, n * n * sizeof(double2)) != cudaSuccess || cudaMalloc(&V, n * n * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&T1, n * n * sizeof(double2)) != cudaSuccess || cudaMalloc(&perm_d, n * sizeof(int)) != cudaSuccess) {
+  if (dev_alloc(c, &ev, n_qp * sizeof(double)) != cudaSuccess || dev_alloc(c, &dots, 4 * n * sizeof(double)) != cudaSuccess ||
+      dev_alloc(c, &H, n * n * sizeof(double2)) != cudaSuccess || dev_alloc(c, &V, n * n * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &T1, n * n * sizeof(double2)) != cudaSuccess || dev_alloc(c, &perm_d, n * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     rc = set_err(c, FBSE_ERR_OOM, "fbse_bse_solve");
   }
@@ -894,8 +889,8 @@ int fbse_bse_dipoles(fbse_ctx *c, const double *psi_qp, const double *gx, const 
   double *dg = nullptr;
   double2 *mu = nullptr;
   int rc = FBSE_OK;
-  if (cudaMalloc(&dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&mu, n_h * n_e * 3 * sizeof(double2)) != cudaSuccess) {
+  if (dev_alloc(c, &dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess ||
+      dev_alloc(c, &mu, n_h * n_e * 3 * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
     if (dg) cudaFree(dg);
     return set_err(c, FBSE_ERR_OOM, "fbse_bse_dipoles");
@@ -938,10 +933,10 @@ int fbse_bse_mag_dipoles(fbse_ctx *c, const double *psi_qp, const double *gx, co
   double2 *dk3 = nullptr, *P = nullptr, *work = nullptr, *m = nullptr;
   double *dg = nullptr;
   int rc = FBSE_OK;
-  if (cudaMalloc(&dk3, 3 * N * sizeof(double2)) != cudaSuccess || cudaMalloc(&P, 3 * nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&work, nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&m, n_h * n_e * 3 * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess) {
+  if (dev_alloc(c, &dk3, 3 * N * sizeof(double2)) != cudaSuccess || dev_alloc(c, &P, 3 * nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &work, nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &m, n_h * n_e * 3 * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     rc = set_err(c, FBSE_ERR_OOM, "fbse_bse_mag_dipoles");
   }
@@ -1001,11 +996,11 @@ int fbse_bse_qp_ang_mom(fbse_ctx *c, const double *psi_qp, const double *gx, con
   double2 *dk3 = nullptr, *P = nullptr, *Lp = nullptr, *L2 = nullptr, *work = nullptr, *dots = nullptr;
   double *dg = nullptr;
   int rc = FBSE_OK;
-  if (cudaMalloc(&dk3, 3 * N * sizeof(double2)) != cudaSuccess || cudaMalloc(&P, 3 * nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&Lp, 3 * nsg * sizeof(double2)) != cudaSuccess || cudaMalloc(&L2, nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&work, nsg * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&dots, nmax * 8 * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess) {
+  if (dev_alloc(c, &dk3, 3 * N * sizeof(double2)) != cudaSuccess || dev_alloc(c, &P, 3 * nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &Lp, 3 * nsg * sizeof(double2)) != cudaSuccess || dev_alloc(c, &L2, nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &work, nsg * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &dots, nmax * 8 * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &dg, (c->nx + c->ny + c->nz) * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     rc = set_err(c, FBSE_ERR_OOM, "fbse_bse_qp_ang_mom");
   }
@@ -1091,7 +1086,7 @@ int fbse_bse_optical(fbse_ctx *c, const double *coeff, const double *mu_pairs_ho
     return c ? set_err(c, FBSE_ERR_ARG, "fbse_bse_optical: bad arguments") : FBSE_ERR_ARG;
   const long n = n_h * n_e;
   double2 *mu = nullptr;
-  if (cudaMalloc(&mu, 2 * n * 3 * sizeof(double2)) != cudaSuccess) {
+  if (dev_alloc(c, &mu, 2 * n * 3 * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, FBSE_ERR_OOM, "fbse_bse_optical");
   }

@@ -215,6 +215,22 @@ inline void release(fbse_ctx *c, int slot)
   c->cache[slot] = nullptr;
   c->cache_bytes[slot] = 0;
 }
+// device memory for the context: the tensor-core products' scratch, kept between calls
+// and idle outside them, goes back before an allocation is given up
+template <typename T> inline cudaError_t dev_alloc(fbse_ctx *c, T **p, size_t bytes)
+{
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess && c->cache[kSlotTc]) {
+    cudaGetLastError();
+    release(c, kSlotTc);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+  }
+  return e;
+}
 // reads (and clears) the device error flags of the kernels with bounded waits
 int check_dev_status(fbse_ctx *c);
 

@@ -179,9 +179,9 @@ static int launch_newton_acc(fbse_ctx *c, const C<T> *ring, long j0, int nk, con
 }
 
 // ring length: fbse_tuning.newton_ring slots (128 by default), halved while
-// the ring would take more than 40% of the free device memory (the ring the
-// context already holds counts as free), at most ncheby.  The FP32 block sums
-// of the accumulation depend on it.
+// the ring would take more than 40% of the free device memory (the ring and the
+// tensor-core scratch that the context already holds count as free), at most
+// ncheby.  The FP32 block sums of the accumulation depend on it.
 static long ring_slots(fbse_ctx *c, long ncheby, size_t slot_bytes)
 {
   long K = c->tune.newton_ring > 0 ? std::min<long>(c->tune.newton_ring, kMaxRing) : kMaxRing;
@@ -190,7 +190,7 @@ static long ring_slots(fbse_ctx *c, long ncheby, size_t slot_bytes)
     cudaGetLastError();
     free_b = 0;
   }
-  free_b += c->cache_bytes[kSlotRing];
+  free_b += c->cache_bytes[kSlotRing] + c->cache_bytes[kSlotTc];
   while (K > 8 && (double)K * slot_bytes > 0.4 * (double)free_b) K /= 2;
   return ncheby < K ? ncheby : K;
 }
@@ -262,7 +262,7 @@ static int newton_filter_t(fbse_ctx *c, const double *zn, const double *an, long
   void *ring = nullptr;
   if ((rc = newton_ring_t<T>(c, ncheby, nstart, &K, &ring))) return rc;
   double *a_dev = nullptr;
-  if (cudaMalloc(&a_dev, are.size() * sizeof(double)) != cudaSuccess) {
+  if (dev_alloc(c, &a_dev, are.size() * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, FBSE_ERR_OOM, "newton coefficients");
   }
@@ -447,7 +447,7 @@ int normalize_all(fbse_ctx *c, double *psitot, long n, double *norms)
   int rc = ensure(c, (void **)&c->red, &c->red_bytes, (size_t)n * kRedBlocks * 2 * sizeof(double));
   if (rc) return rc;
   double *d = nullptr;
-  if (cudaMalloc(&d, n * 2 * sizeof(double)) != cudaSuccess) return set_err(c, FBSE_ERR_OOM, "norms");
+  if (dev_alloc(c, &d, n * 2 * sizeof(double)) != cudaSuccess) return set_err(c, FBSE_ERR_OOM, "norms");
   std::vector<double> h(2 * n), f(n);
   do {
     FBSE_COUNT(2); k_sumsq<<<dim3(kRedBlocks, (unsigned)n), 256, 0, c->stream>>>(psitot, stlen, c->red);
@@ -481,7 +481,7 @@ static int energy_all_t(fbse_ctx *c, const double *psitot, long n, double *ene, 
   // process in chunks of working states to bound scratch
   const long chunk = nw < 16 ? nw : 16;
   C<T> *buf = nullptr;
-  if (cudaMalloc(&buf, 2 * chunk * len * sizeof(C<T>)) != cudaSuccess) return set_err(c, FBSE_ERR_OOM, "energy_all");
+  if (dev_alloc(c, &buf, 2 * chunk * len * sizeof(C<T>)) != cudaSuccess) return set_err(c, FBSE_ERR_OOM, "energy_all");
   std::vector<double> h(2 * chunk), h2(2 * chunk);
   int rc = FBSE_OK;
   const long stlen = (long)(c->is_complex + 1) * len;
@@ -603,8 +603,8 @@ static int energy_range_t(fbse_ctx *c, long seed, long max_iter, double *emin_ou
   const long len = (long)c->nspin * c->ngrid;
   C<T> *buf = nullptr;  // phi, h
   double *hd = nullptr;
-  if (cudaMalloc(&buf, 2 * len * sizeof(C<T>)) != cudaSuccess) return set_err(c, FBSE_ERR_OOM, "energy range");
-  if (cudaMalloc(&hd, len * 2 * sizeof(double)) != cudaSuccess) { cudaFree(buf); return set_err(c, FBSE_ERR_OOM, "energy range"); }
+  if (dev_alloc(c, &buf, 2 * len * sizeof(C<T>)) != cudaSuccess) return set_err(c, FBSE_ERR_OOM, "energy range");
+  if (dev_alloc(c, &hd, len * 2 * sizeof(double)) != cudaSuccess) { cudaFree(buf); return set_err(c, FBSE_ERR_OOM, "energy range"); }
   C<T> *phi = buf, *h = buf + len;
   std::vector<double> host(2 * len);
   int rc = FBSE_OK;

@@ -73,7 +73,7 @@ extern "C" int fbse_filter_job(fbse_ctx *c, const double *zn, const double *an, 
                           cudaHostGetDevicePointer(&hdev, psi_host, 0) == cudaSuccess && hdev;
       if (!mapped) cudaGetLastError();
       int *dsel = nullptr;
-      if (mapped && cudaMalloc(&dsel, w * sizeof(int)) == cudaSuccess &&
+      if (mapped && dev_alloc(c, &dsel, w * sizeof(int)) == cudaSuccess &&
           cudaMemcpyAsync(dsel, sel.data(), w * sizeof(int), cudaMemcpyHostToDevice, c->stream) == cudaSuccess) {
         k_gather_states<<<4096, 256, 0, c->stream>>>(reinterpret_cast<const double2 *>(df), dsel, w, stlen / 2,
                                                      reinterpret_cast<double2 *>(hdev));

@@ -834,11 +834,7 @@ static int ortho_diag_sigma_t(fbse_ctx *c, double *psitot, long n_, long *n_kept
   const long kchunk = (L + nchunk - 1) / nchunk;
   const int nrb = (int)((L + 127) / 128);
   auto alloc = [&](void **p, size_t b) -> bool {
-    if (cudaMalloc(p, b) == cudaSuccess) return true;
-    cudaGetLastError();
-    release(c, kSlotTc);  // an earlier product's scratch
-    if (cudaMalloc(p, b) == cudaSuccess) return true;
-    cudaGetLastError();
+    if (dev_alloc(c, p, b) == cudaSuccess) return true;
     rc = set_err(c, FBSE_ERR_OOM, "ortho/diag scratch");
     return false;
   };
@@ -1106,7 +1102,7 @@ int gram_slab(fbse_ctx *c, const double *A, long na, const double *B, long nb, l
     // not one of the context's kept buffers: a captured graph may hold their addresses
     double2 *o = nullptr;
     int rx = FBSE_OK;
-    if (cudaMalloc(&o, (size_t)na * nb * sizeof(double2)) != cudaSuccess) {
+    if (dev_alloc(c, &o, (size_t)na * nb * sizeof(double2)) != cudaSuccess) {
       cudaGetLastError();
       rx = FBSE_ERR_OOM;
     }
@@ -1122,8 +1118,8 @@ int gram_slab(fbse_ctx *c, const double *A, long na, const double *B, long nb, l
   const int nchunk = (int)std::min<long>(std::max<long>(1, len / 8192), 256);
   const long kchunk = (len + nchunk - 1) / nchunk;
   double2 *part = nullptr, *sum = nullptr;
-  if (cudaMalloc(&part, (size_t)nchunk * na * nb * sizeof(double2)) != cudaSuccess ||
-      cudaMalloc(&sum, (size_t)na * nb * sizeof(double2)) != cudaSuccess) {
+  if (dev_alloc(c, &part, (size_t)nchunk * na * nb * sizeof(double2)) != cudaSuccess ||
+      dev_alloc(c, &sum, (size_t)na * nb * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
     if (part) cudaFree(part);
     return set_err(c, FBSE_ERR_OOM, "fbse_gram: scratch");
@@ -1151,7 +1147,7 @@ int rotate_slab(fbse_ctx *c, const double *A, long na, const double *C_host, lon
   const long stride = (long)(c->is_complex + 1) * L;
   if (na < 1 || k < 1 || off < 0 || len < 1 || off + len > L) return set_err(c, FBSE_ERR_ARG, "fbse_rotate: sizes");
   double2 *Cd = nullptr;
-  if (cudaMalloc(&Cd, (size_t)na * k * sizeof(double2)) != cudaSuccess) {
+  if (dev_alloc(c, &Cd, (size_t)na * k * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, FBSE_ERR_OOM, "fbse_rotate: coefficients");
   }

@@ -857,7 +857,7 @@ static int residual_dev(fbse_ctx *c, const double *psi, long n, const double *e_
   const size_t wbytes = (c->precision == FBSE_MIXED ? sizeof(float2) : sizeof(double2)) * (size_t)len;
   const long chunk = 16;
   void *w0 = nullptr;
-  if (cudaMalloc(&w0, 2 * chunk * wbytes) != cudaSuccess) {
+  if (dev_alloc(c, &w0, 2 * chunk * wbytes) != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, FBSE_ERR_OOM, "residual: H psi scratch");
   }
@@ -885,7 +885,7 @@ static int residual_dev(fbse_ctx *c, const double *psi, long n, const double *e_
 static int residual_host_e(fbse_ctx *c, const double *psi, long n, const double *e_host, double *r)
 {
   double *ed = nullptr;
-  if (cudaMalloc(&ed, n * sizeof(double)) != cudaSuccess) {
+  if (dev_alloc(c, &ed, n * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, FBSE_ERR_OOM, "residual: energies");
   }
@@ -950,7 +950,7 @@ int fbse_precond_create(fbse_ctx *c, fbse_precond **out, const float *weights, l
   P->c = c;
   const size_t nw = FBSE_PRECOND_NWEIGHTS;
   void *m = nullptr;
-  if (cudaMalloc(&m, nw * sizeof(float) * 5 + nw * sizeof(double) + 2 * pc::tcc::kWBytes) != cudaSuccess) {
+  if (dev_alloc(c, &m, nw * sizeof(float) * 5 + nw * sizeof(double) + 2 * pc::tcc::kWBytes) != cudaSuccess) {
     cudaGetLastError();
     delete P;
     return set_err(c, FBSE_ERR_OOM, "fbse_precond_create");
