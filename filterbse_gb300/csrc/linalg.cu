@@ -233,12 +233,12 @@ int zgemm_dev(fbse_ctx *c, int m, int p, int k, const double2 *A, int lda, bool 
 // one buffer and writes every element to another, and each tile of 8 x 8 blocks (or
 // 8 pairs x 32 rows of V) computes the rotations of its own 16 pairs.  Tiles of 64
 // threads spread the FP64 work (2 lanes per clock and SM) over every SM from n = 128
-// on.  Measured per round against two barriers and a thread per block of the whole
-// matrix: n = 128 12.5 -> 6.6 us, n = 196 12.7 -> 6.9 us, n = 115 real 12.4 -> 6.6 us.
+// on.  Larger matrices share the rotations behind a second barrier (jacobi_eig_dev).
+// Measured per round against two barriers and a thread per block of the whole matrix:
+// n = 128 12.5 -> 6.6 us, n = 196 12.7 -> 6.9 us, n = 115 real 12.4 -> 6.6 us.
 // ---------------------------------------------------------------------------
-struct Rot {
+struct __align__(16) Rot {
   double cs, sn, pr, pi;  // U = D J:  U_pp = cs, U_pq = sn, U_qp = -sn e^{-i phi}, U_qq = cs e^{-i phi}
-  int p, q;
 };
 
 __device__ __forceinline__ void rr_pair(int r, int slot, int m, int &p, int &q)
@@ -253,7 +253,7 @@ __device__ __forceinline__ void rr_pair(int r, int slot, int m, int &p, int &q)
 // the rotation that zeroes the pair's off-diagonal element
 __device__ __forceinline__ Rot pair_rotation(const double2 *__restrict__ A, int n, int p, int q)
 {
-  Rot R{1.0, 0.0, 1.0, 0.0, p, q};
+  Rot R{1.0, 0.0, 1.0, 0.0};
   if (q < n) {
     const double app = __ldcg(&A[(long)p * n + p]).x, aqq = __ldcg(&A[(long)q * n + q]).x;
     const double2 apq = __ldcg(&A[(long)p * n + q]);
@@ -293,12 +293,14 @@ constexpr int kJT = 8, kJRows = 32, kJThreads = 64;  // pairs per tile side, V r
 
 // REAL: every imaginary part is zero and stays zero.  off[0..1]: off-diagonal and
 // diagonal sums of squares, off[2]: nonzero when a barrier gave up, then the CTAs'
-// partial sums.  count0: barriers of earlier launches on this counter.
+// partial sums.  count0: arrivals of earlier launches on this counter.  rots: room for
+// the round's m / 2 rotations when they are formed once, behind a barrier of their own,
+// else null.
 template <bool REAL>
 __global__ void __launch_bounds__(kJThreads) k_jacobi_sweep(double2 *__restrict__ A0, double2 *__restrict__ A1,
                                                             double2 *__restrict__ V, int n, int m,
-                                                            unsigned *__restrict__ counter, unsigned count0,
-                                                            double *__restrict__ off)
+                                                            Rot *__restrict__ rots, unsigned *__restrict__ counter,
+                                                            unsigned count0, double *__restrict__ off)
 {
   const int half = m / 2, T = (half + kJT - 1) / kJT, TV = (n + kJRows - 1) / kJRows;
   const int na = T * T, ntile = na + T * TV;
@@ -321,6 +323,18 @@ __global__ void __launch_bounds__(kJThreads) k_jacobi_sweep(double2 *__restrict_
   for (int r = 0; r < m - 1; r++) {
     const double2 *src = (r & 1) ? A1 : A0;
     double2 *dst = (r & 1) ? A0 : A1;
+    if (rots) {
+      for (int s = blockIdx.x * kJThreads + tid; s < half; s += gridDim.x * kJThreads) {
+        int p, q;
+        rr_pair(r, s, m, p, q);
+        rots[s] = pair_rotation(src, n, p, q);
+      }
+      gen += gridDim.x;
+      if (!grid_barrier(counter, gen)) {
+        if (tid == 0) off[2] = 1.0;
+        return;
+      }
+    }
     for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
       const bool on_a = tile < na;
       // tiles of pairs; V: pairs tb, rows ta
@@ -353,9 +367,15 @@ __global__ void __launch_bounds__(kJThreads) k_jacobi_sweep(double2 *__restrict_
       if (tid < 2 * kJT) {
         const int s = (tid < kJT ? ta * kJT : tb * kJT - kJT) + tid;
         if (s < half && (on_a || tid >= kJT)) {
-          int p, q;
-          rr_pair(r, s, m, p, q);
-          rot[tid] = pair_rotation(src, n, p, q);
+          if (rots) {
+            const double2 *t = reinterpret_cast<const double2 *>(rots + s);
+            const double2 j = __ldcg(t), phase = __ldcg(t + 1);
+            rot[tid] = Rot{j.x, j.y, phase.x, phase.y};
+          } else {
+            int p, q;
+            rr_pair(r, s, m, p, q);
+            rot[tid] = pair_rotation(src, n, p, q);
+          }
         }
       }
       __syncthreads();
@@ -455,16 +475,27 @@ int jacobi_eig_dev(fbse_ctx *c, double2 *A, double2 *V, int n, std::vector<doubl
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kJThreads, 0);
   const long T = (m / 2 + kJT - 1) / kJT, tiles = T * T + T * ((n + kJRows - 1) / kJRows);
-  // a tile per CTA, up to four CTAs per SM (more only lengthen the barrier)
-  const int blocks = (int)std::min<long>(std::max<long>(1, tiles), (long)nsm * std::min(4, std::max(1, per_sm)));
+  // a tile per CTA, up to four CTAs per SM (more only lengthen the barrier; eight gain 3%
+  // at n = 1600 and lose 10% at 784)
+  const int most = nsm * std::min(4, std::max(1, per_sm));
+  const int blocks = (int)std::min<long>(std::max<long>(1, tiles), most);
+  // A tile that forms its 16 rotations spends two thirds of its FP64 time on them, which
+  // is hidden behind the barrier while every tile has a CTA and SM time to itself (n up to
+  // 320).  With more tiles than CTAs the rotations are formed once, behind a second
+  // barrier: eigensolve of n = 360 52 -> 46 ms, 784 394 -> 259, 1600 3.56 -> 2.03 s (0.33
+  // and 2.43 s with a thread per block and two barriers), 3360 18 s (22).  The values are
+  // the same.
+  const bool table = tiles > most;
   // the second buffer of A, the norms and their partials, the barrier's counter,
   // kept in the context between calls
-  const size_t a_bytes = (size_t)n * n * sizeof(double2), off_bytes = (3 + 2 * (size_t)blocks) * sizeof(double);
+  const size_t a_bytes = (size_t)n * n * sizeof(double2), rot_bytes = table ? m / 2 * sizeof(Rot) : 0;
+  const size_t off_bytes = (3 + 2 * (size_t)blocks) * sizeof(double);
   void *scratch = nullptr;
-  int rc = cached(c, kSlotJacobi, a_bytes + off_bytes + 16, &scratch);
+  int rc = cached(c, kSlotJacobi, a_bytes + rot_bytes + off_bytes + 16, &scratch);
   if (rc) return rc;
   double2 *A1 = static_cast<double2 *>(scratch), *cur = A, *other = A1;
-  double *off = reinterpret_cast<double *>(static_cast<char *>(scratch) + a_bytes);
+  Rot *rots = table ? reinterpret_cast<Rot *>(A1 + (size_t)n * n) : nullptr;
+  double *off = reinterpret_cast<double *>(static_cast<char *>(scratch) + a_bytes + rot_bytes);
   unsigned *counter = reinterpret_cast<unsigned *>(off + 3 + 2 * blocks), count = 0;
   FBSE_CUDA(c, cudaMemsetAsync(off, 0, off_bytes + 16, c->stream));
   FBSE_COUNT(1); k_identity<<<256, 256, 0, c->stream>>>(V, n);
@@ -472,12 +503,13 @@ int jacobi_eig_dev(fbse_ctx *c, double2 *A, double2 *V, int n, std::vector<doubl
   bool conv = (n < 2);
   for (int sweep = 0; sweep < 60 && !conv; sweep++) {
     int mm = m;
-    void *args[] = {&cur, &other, &V, &n, &mm, &counter, &count, &off};
+    void *args[] = {&cur, &other, &V, &n, &mm, &rots, &counter, &count, &off};
     FBSE_COUNT(1); if (cudaLaunchCooperativeKernel(kernel, blocks, kJThreads, args, 0, c->stream) != cudaSuccess) {
       rc = set_err(c, FBSE_ERR_CUDA, std::string("jacobi launch: ") + cudaGetErrorString(cudaGetLastError()));
       break;
     }
-    count += (unsigned)m * (unsigned)blocks;  // m - 1 rounds and the norms
+    // m - 1 rounds, twice with the table, and the norms
+    count += (unsigned)(table ? 2 * m - 1 : m) * (unsigned)blocks;
     if ((m - 1) & 1) std::swap(cur, other);
     if (cudaMemcpyAsync(h, off, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) {
