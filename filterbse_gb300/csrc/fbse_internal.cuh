@@ -156,7 +156,7 @@ struct fbse_ctx {
   int tc_poisoned = 0;  // a tensor-core wait timed out: MMAs may still be in flight, the path is refused
   // the Rayleigh-Ritz step (ortho_diag_sigma) is running: H psi takes the mixed-radix
   // FFT kernels on every axis that the register-resident ones do not, and the
-  // gather a warp per state
+  // gather a warp per state; the autotuner's problems of these kernels say so
   int steady = 0;
   int nsm = 0;          // multiprocessors of the device (queried on first use)
   // large buffers kept between calls (grown on demand, freed by fbse_destroy):

@@ -952,9 +952,12 @@ static int fft_op_apply(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, long
       std::vector<long> cands{nblk};
       for (long v : {16L, 8L, 4L, 2L})
         if (v < nblk) cands.push_back(v);
+      // the Rayleigh-Ritz step runs other kernels on all but these grids
+      const bool other = c->steady && !(fast_axis_ok(c, c->nx) && fast_axis_ok(c, c->ny) && fast_axis_ok(c, c->nz));
       const std::string prob = std::string(sizeof(T) == 4 ? "fp32" : "fp64") + " grid=" + std::to_string(c->nx) +
                                "x" + std::to_string(c->ny) + "x" + std::to_string(c->nz) +
-                               " blocks=" + std::to_string(nblk) + (kq ? " convolution" : " kinetic");
+                               " blocks=" + std::to_string(nblk) + (kq ? " convolution" : " kinetic") +
+                               (other ? " Rayleigh-Ritz" : "");
       int rc = autotune(c, "fft blocks per launch", prob, cands,
                         [&](long v) { return fft_op_chunked<T>(c, in, out, work, nblk, a, b, with_v, kq, v); }, &cb);
       if (rc) return rc;

@@ -635,7 +635,7 @@ static int proj_gather(fbse_ctx *c, const C<T> *in, long nstates, long st0 = 0)
   const ProjView<T> pv = view<T>(c);
   const std::string prob = std::string(sizeof(T) == 4 ? "fp32" : "fp64") + " states=" + std::to_string(nstates) +
                            " atoms=" + std::to_string(p.nat) + " points=" + std::to_string(p.ncov) +
-                           (c->so ? " SO" : "") + (c->nl ? " NL" : "");
+                           (c->so ? " SO" : "") + (c->nl ? " NL" : "") + (c->steady ? " Rayleigh-Ritz" : "");
   // points per lane per iteration (the same sums in the same order for every
   // choice); the gather writes only coef, so candidates run in place
   long gu = c->tune.gather_points;
