@@ -938,9 +938,10 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
 }
 
 // blocks per launch sequence: fixed by fbse_tuning.fft_chunk_blocks or
-// autotuned (every block is transformed by the same kernels either way; a
-// smaller chunk keeps its intermediate passes in L2, a larger one fills the
-// GPU better)
+// autotuned (every block gets the same bits either way: the FP64 two-factor plane
+// and line kernels, between which a launch's blocks decide, share their stages;
+// a smaller chunk keeps its intermediate passes in L2, a larger one fills the GPU
+// better)
 template <typename T>
 static int fft_op_apply(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, long nblk, double a, double b,
                         int with_v, const double2 *kq)

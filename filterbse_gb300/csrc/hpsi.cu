@@ -732,8 +732,8 @@ int hpsi_apply(fbse_ctx *c, const C<T> *in, C<T> *out, long nstates, double a, d
   // with the projectors on and input and output apart, the batch runs as
   // parts (two by default) on the context's streams, each gather -> FFT
   // passes -> scatter, so that one part's projector kernels (latency bound)
-  // and tail waves overlap the other parts' kernels; every state sees the
-  // same kernels either way
+  // and tail waves overlap the other parts' kernels; every state gets the same
+  // bits either way (fft.cu's two_planes may take other kernels for fewer blocks)
   const char *i0 = reinterpret_cast<const char *>(in), *o0 = reinterpret_cast<const char *>(out);
   const bool apart = i0 + need <= o0 || o0 + need <= i0;
   const long parts = std::min<long>(nstates, c->tune.hpsi_streams == 0 ? 2 : c->tune.hpsi_streams);
