@@ -46,12 +46,9 @@ struct Stages {
   int n;
   int nst;
   int radix[kMaxStages];
-  int big;   // 1 when a radix exceeds the register limit (pass_big)
-  int most;  // butterflies of a line in the register pass that has most
+  int big;  // 1 when a radix exceeds the register limit (needs a scratch line)
 };
 constexpr int kLineThreads = 256, kPlaneThreads = 1024;
-// the line kernels keep a second set of lines for passes that are not in place
-__host__ __device__ inline bool needs_scratch(const Stages &s) { return s.big || s.most > kLineThreads; }
 
 constexpr int kRegMax = 8;  // odd radices above this take the scratch pass
 
@@ -167,14 +164,20 @@ static Stages stages_of(const AxisPlan &p)
   s.n = p.n;
   s.nst = p.nst;
   s.big = 0;
-  s.most = 0;
   for (int i = 0; i < kMaxStages; i++) {
     s.radix[i] = p.radix[i];
-    if (i >= p.nst) continue;
-    if (p.radix[i] > kRegMax && p.radix[i] != 16) s.big = 1;
-    else s.most = std::max(s.most, p.n / p.radix[i]);
+    if (i < p.nst && p.radix[i] > kRegMax && p.radix[i] != 16) s.big = 1;
   }
   return s;
+}
+
+// butterflies of a line in the register pass that has most
+static int most_butterflies(const AxisPlan &p)
+{
+  int most = 0;
+  for (int i = 0; i < p.nst; i++)
+    if (p.radix[i] <= kRegMax || p.radix[i] == 16) most = std::max(most, p.n / p.radix[i]);
+  return most;
 }
 
 template <typename T> static const C<T> *roots(const AxisPlan &p);
@@ -264,15 +267,18 @@ __device__ __noinline__ void pass_wide(C<T> *buf, int es, int ls, int n, int L, 
 // ---------------------------------------------------------------------------
 // one in-place Stockham pass of radix R over L lines (element i of line c at
 // buf[c * ls + i * es]); lanes take consecutive lines at one butterfly index.
-// scr: needed where a line has more butterflies than the CTA threads (pass_wide)
+// WIDE: a line may have more butterflies than the CTA threads (pass_wide, with scr);
+// kernels without it keep the registers that its calls would take
 // ---------------------------------------------------------------------------
-template <typename T, int R>
+template <typename T, int R, bool WIDE>
 __device__ __forceinline__ void pass_reg(C<T> *buf, int es, int ls, int n, int L, int Ns, const C<T> *__restrict__ tw,
                                       bool inv, C<T> *scr)
 {
-  if (n / R > (int)blockDim.x) {
-    pass_wide<T, R>(buf, es, ls, n, L, Ns, tw, inv, scr);
-    return;
+  if constexpr (WIDE) {
+    if (n / R > (int)blockDim.x) {
+      pass_wide<T, R>(buf, es, ls, n, L, Ns, tw, inv, scr);
+      return;
+    }
   }
   constexpr int kMaxE = R;                              // one butterfly per thread per round
   constexpr int BMAX = (kMaxE / R) > 0 ? kMaxE / R : 1;
@@ -417,21 +423,31 @@ __device__ __noinline__ void pass_big(C<T> *buf, int es, int ls, int n, int L, i
   __syncthreads();
 }
 
-template <typename T>
+// the passes a kernel holds: register radices in place; those and pass_big; every one.
+// A call costs registers whether it is taken or not, so only the line kernels of such
+// axes have them
+enum Passes { kInPlace, kBig, kWide };
+// CTAs per SM of a line kernel: 64 registers a thread do for the register radices (16 FP32
+// states of 120 x 112 x 60 997 us, with 128 registers 1109) and make pass_big spill
+template <Passes PASSES> constexpr int kLineCtas = PASSES == kInPlace ? 4 : 2;
+
+template <typename T, Passes PASSES>
 __device__ void fft_lines(C<T> *buf, int es, int ls, int L, const Stages &st, const C<T> *tw, bool inv, C<T> *scr)
 {
   int Ns = 1;
   for (int s = 0; s < st.nst; s++) {
     const int R = st.radix[s];
     switch (R) {
-      case 2: pass_reg<T, 2>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
-      case 3: pass_reg<T, 3>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
-      case 4: pass_reg<T, 4>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
-      case 5: pass_reg<T, 5>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
-      case 7: pass_reg<T, 7>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
-      case 8: pass_reg<T, 8>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
-      case 16: pass_reg<T, 16>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
-      default: pass_big<T>(buf, es, ls, st.n, L, R, Ns, tw, inv, scr); break;
+      case 2: pass_reg<T, 2, PASSES == kWide>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 3: pass_reg<T, 3, PASSES == kWide>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 4: pass_reg<T, 4, PASSES == kWide>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 5: pass_reg<T, 5, PASSES == kWide>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 7: pass_reg<T, 7, PASSES == kWide>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 8: pass_reg<T, 8, PASSES == kWide>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      case 16: pass_reg<T, 16, PASSES == kWide>(buf, es, ls, st.n, L, Ns, tw, inv, scr); break;
+      default:
+        if constexpr (PASSES != kInPlace) pass_big<T>(buf, es, ls, st.n, L, R, Ns, tw, inv, scr);
+        break;
     }
     Ns *= R;
   }
@@ -463,13 +479,13 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) k_fft_plane(const C<T> *__re
   for (int t = threadIdx.x; t < npl; t += blockDim.x) P[(t / nx) * nxp + t % nx] = in[base + t];
   __syncthreads();
   if (MODE == 0) {
-    fft_lines<T>(P, 1, nxp, ny, sx, twx, false, nullptr);  // rows
-    fft_lines<T>(P, nxp, 1, nx, sy, twy, false, nullptr);  // columns
+    fft_lines<T, kInPlace>(P, 1, nxp, ny, sx, twx, false, nullptr);  // rows
+    fft_lines<T, kInPlace>(P, nxp, 1, nx, sy, twy, false, nullptr);  // columns
 #pragma unroll 8
     for (int t = threadIdx.x; t < npl; t += blockDim.x) out[base + t] = P[(t / nx) * nxp + t % nx];
   } else {
-    fft_lines<T>(P, nxp, 1, nx, sy, twy, true, nullptr);
-    fft_lines<T>(P, 1, nxp, ny, sx, twx, true, nullptr);
+    fft_lines<T, kInPlace>(P, nxp, 1, nx, sy, twy, true, nullptr);
+    fft_lines<T, kInPlace>(P, 1, nxp, ny, sx, twx, true, nullptr);
 #pragma unroll 8
     for (int t = threadIdx.x; t < npl; t += blockDim.x) {
       const long g = base + t;
@@ -491,8 +507,8 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) k_fft_plane(const C<T> *__re
 // x line pass (line path): L contiguous lines per CTA, line stride n|1.
 // EPI = 1: fused out = a (kin + V phi) + b phi.
 // ---------------------------------------------------------------------------
-template <typename T, int EPI>
-__global__ void __launch_bounds__(kLineThreads, 2) k_fft_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages st,
+template <typename T, int EPI, Passes PASSES>
+__global__ void __launch_bounds__(kLineThreads, kLineCtas<PASSES>) k_fft_x(const C<T> *__restrict__ in, C<T> *__restrict__ out, Stages st,
                                                const C<T> *__restrict__ twg, long nlines, int L, bool inv,
                                                const C<T> *__restrict__ phi, const T *__restrict__ pot, long ngrid,
                                                T ca, T cb)
@@ -501,7 +517,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_fft_x(const C<T> *__restric
   const int n = st.n, np = n | 1;
   C<T> *tw = reinterpret_cast<C<T> *>(smem_raw);
   C<T> *A = tw + n;
-  C<T> *S = A + (long)L * np;  // scratch (needs_scratch)
+  C<T> *S = A + (long)L * np;  // scratch of passes that are not in place
   for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];
   const long line0 = (long)blockIdx.x * L;
   const int nl = (int)min((long)L, nlines - line0);
@@ -509,7 +525,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_fft_x(const C<T> *__restric
 #pragma unroll 8
   for (int t = threadIdx.x; t < nl * n; t += blockDim.x) A[(t / n) * np + t % n] = in[off + t];
   __syncthreads();
-  fft_lines<T>(A, 1, np, nl, st, tw, inv, needs_scratch(st) ? S : nullptr);
+  fft_lines<T, PASSES>(A, 1, np, nl, st, tw, inv, PASSES != kInPlace ? S : nullptr);
 #pragma unroll 8
   for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
     C<T> v = A[(t / n) * np + t % n];
@@ -534,8 +550,8 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_fft_x(const C<T> *__restric
 // base = (o / cnt) * s1 + (o % cnt) * s2 + xt * TX.
 // KMUL: forward, multiply by the kinetic factor, inverse (z pass only).
 // ---------------------------------------------------------------------------
-template <typename T, bool KMUL>
-__global__ void __launch_bounds__(kLineThreads, 2) k_fft_cols(C<T> *__restrict__ data, Stages st, const C<T> *__restrict__ twg,
+template <typename T, bool KMUL, Passes PASSES>
+__global__ void __launch_bounds__(kLineThreads, kLineCtas<PASSES>) k_fft_cols(C<T> *__restrict__ data, Stages st, const C<T> *__restrict__ twg,
                                                   long es, int nxc, int TX, int nxt, long cnt, long s1, long s2,
                                                   bool inv, KinArgs ka)
 {
@@ -543,7 +559,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_fft_cols(C<T> *__restrict__
   const int n = st.n;
   C<T> *tw = reinterpret_cast<C<T> *>(smem_raw);
   C<T> *A = tw + n;
-  C<T> *S = A + (long)TX * n;  // scratch (needs_scratch)
+  C<T> *S = A + (long)TX * n;  // scratch of passes that are not in place
   for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twg[t];
   const long o = blockIdx.x / nxt;
   const int xt = blockIdx.x % nxt;
@@ -556,7 +572,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_fft_cols(C<T> *__restrict__
     A[i * L + cc] = data[base + (long)i * es + cc];
   }
   __syncthreads();
-  fft_lines<T>(A, L, 1, L, st, tw, KMUL ? false : inv, needs_scratch(st) ? S : nullptr);
+  fft_lines<T, PASSES>(A, L, 1, L, st, tw, KMUL ? false : inv, PASSES != kInPlace ? S : nullptr);
   if (KMUL) {
     const int jy = (int)(o % cnt);
     if (ka.kq) {
@@ -573,7 +589,7 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_fft_cols(C<T> *__restrict__
       }
     }
     __syncthreads();
-    fft_lines<T>(A, L, 1, L, st, tw, true, needs_scratch(st) ? S : nullptr);
+    fft_lines<T, PASSES>(A, L, 1, L, st, tw, true, PASSES != kInPlace ? S : nullptr);
   }
 #pragma unroll 8
   for (int t = threadIdx.x; t < n * L; t += blockDim.x) {
@@ -609,6 +625,16 @@ static int max_smem()
   return v;
 }
 
+// f with the kind of passes that an axis needs.  Tiles of which an SM holds two at most
+// take the kernels with 128 registers as well (16 FP32 states of 512 x 40 x 64 1649 ->
+// 1540 us)
+template <typename F> static int with_passes(bool big, bool wide, size_t smem, F f)
+{
+  if (wide) return f(std::integral_constant<Passes, kWide>{});
+  if (big || 3 * (smem + 1024) > 228 * 1024) return f(std::integral_constant<Passes, kBig>{});
+  return f(std::integral_constant<Passes, kInPlace>{});
+}
+
 template <typename T>
 static int launch_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv, int epi, const C<T> *phi,
                     const T *pot, T ca, T cb)
@@ -617,20 +643,22 @@ static int launch_x(fbse_ctx *c, const C<T> *in, C<T> *out, long nblk, bool inv,
   const int n = p.n;
   const long nlines = nblk * c->ny * c->nz;
   Stages st = stages_of(p);
+  const bool wide = most_butterflies(p) > kLineThreads;
   int L = 32;
-  while (L > 1 && (size_t)(n + (needs_scratch(st) ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>) > (size_t)max_smem()) L /= 2;
-  const size_t smem = (size_t)(n + (needs_scratch(st) ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>);
+  while (L > 1 && (size_t)(n + (wide || st.big ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>) > (size_t)max_smem()) L /= 2;
+  const size_t smem = (size_t)(n + (wide || st.big ? 2L : 1L) * L * (n | 1)) * sizeof(C<T>);
   const long grid = (nlines + L - 1) / L;
-  if (epi) {
-    FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_x<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_x<T, 1><<<grid, kLineThreads, smem, c->stream>>>(in, out, st, roots<T>(p), nlines, L, inv, phi, pot, c->ngrid, ca, cb);
-  } else {
-    FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_x<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_x<T, 0><<<grid, kLineThreads, smem, c->stream>>>(in, out, st, roots<T>(p), nlines, L, inv, nullptr, nullptr,
-                                                   c->ngrid, T(1), T(0));
-  }
-  FBSE_CHECK_LAUNCH(c);
-  return FBSE_OK;
+  auto go = [&](auto kernel, const C<T> *ph, const T *v, T ea, T eb) -> int {
+    FBSE_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, kLineThreads, smem, c->stream>>>(in, out, st, roots<T>(p), nlines, L, inv, ph, v, c->ngrid, ea, eb);
+    FBSE_CHECK_LAUNCH(c);
+    return FBSE_OK;
+  };
+  auto pick = [&](auto passes) -> int {
+    constexpr Passes P = decltype(passes)::value;
+    return epi ? go(k_fft_x<T, 1, P>, phi, pot, ca, cb) : go(k_fft_x<T, 0, P>, nullptr, nullptr, T(1), T(0));
+  };
+  return with_passes(st.big, wide, smem, pick);
 }
 
 // the z pass's multiplier: the kinetic tables, or the k-space array kq, for x and
@@ -649,9 +677,10 @@ static int launch_cols(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, b
   const int n = p.n;
   const Stages st = stages_of(p);
   int TX = cols_tile((int)c->nx, (int)sizeof(C<T>));
-  auto bytes = [&] { return (size_t)(n + (needs_scratch(st) ? 2L : 1L) * TX * n) * sizeof(C<T>); };
+  const bool wide = most_butterflies(p) > kLineThreads;
+  auto bytes = [&] { return (size_t)(n + (wide || st.big ? 2L : 1L) * TX * n) * sizeof(C<T>); };
   // narrower tiles where a long axis' register passes need the scratch
-  while (!st.big && needs_scratch(st) && TX > 1 && bytes() > (size_t)max_smem()) TX = (TX + 1) / 2;
+  while (!st.big && wide && TX > 1 && bytes() > (size_t)max_smem()) TX = (TX + 1) / 2;
   const int nxt = (int)((c->nx + TX - 1) / TX);
   long es, cnt, s1, s2, nouter;
   if (axis == 1) {  // y lines: outer = block*nz + z
@@ -670,17 +699,17 @@ static int launch_cols(fbse_ctx *c, C<T> *data, long nblk, int axis, bool inv, b
   const size_t smem = bytes();
   if (smem > (size_t)max_smem()) return set_err(c, FBSE_ERR_UNSUPPORTED, "FFT axis too long for shared memory");
   const long grid = nouter * nxt;
-  if (kmul) {
-    FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_cols<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_cols<T, true><<<grid, kLineThreads, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1, s2,
-                                                         inv, ka);
-  } else {
-    FBSE_CUDA(c, cudaFuncSetAttribute(k_fft_cols<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_fft_cols<T, false><<<grid, kLineThreads, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1,
-                                                          s2, inv, ka);
-  }
-  FBSE_CHECK_LAUNCH(c);
-  return FBSE_OK;
+  auto go = [&](auto kernel) -> int {
+    FBSE_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, kLineThreads, smem, c->stream>>>(data, st, roots<T>(p), es, (int)c->nx, TX, nxt, cnt, s1, s2, inv, ka);
+    FBSE_CHECK_LAUNCH(c);
+    return FBSE_OK;
+  };
+  auto pick = [&](auto passes) -> int {
+    constexpr Passes P = decltype(passes)::value;
+    return kmul ? go(k_fft_cols<T, true, P>) : go(k_fft_cols<T, false, P>);
+  };
+  return with_passes(st.big, wide, smem, pick);
 }
 
 template <typename T> static size_t plane_smem(fbse_ctx *c)
@@ -897,7 +926,8 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
   // memory, or y and x lines with the same arithmetic in the same order
   const bool both = !fplane && c->tune.fft_kernels == 0 && !c->steady && c->ax[0].P > 0 && c->ax[1].P > 0;
   const bool lines = two_axis_ok(c, 0) || two_axis_ok(c, 1);
-  const bool plane = !lines && !sx.big && !sy.big && std::max(sx.most, sy.most) <= kPlaneThreads &&
+  const bool plane = !lines && !sx.big && !sy.big &&
+                     std::max(most_butterflies(c->ax[0]), most_butterflies(c->ax[1])) <= kPlaneThreads &&
                      plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;
   // which of x and y the z pass meets in a two-factor transform's order
   const bool xo = both || (!fplane && !plane && two_axis_ok(c, 0));
