@@ -926,7 +926,12 @@ static int fft_op_chunked(fbse_ctx *c, const C<T> *in, C<T> *out, C<T> *work, lo
   // memory, or y and x lines with the same arithmetic in the same order
   const bool both = !fplane && c->tune.fft_kernels == 0 && !c->steady && c->ax[0].P > 0 && c->ax[1].P > 0;
   const bool lines = two_axis_ok(c, 0) || two_axis_ok(c, 1);
-  const bool plane = !lines && !sx.big && !sy.big &&
+  // the mixed-radix planes also beside a two-factor y axis, in FP32, when x has no two
+  // factors and y is short: 1 and 16 states of 512 x 10 x 64 97 and 475 us (lines 159, 475), of
+  // 1024 x 10 x 64 132 and 788 (162, 895), 768 x 20 x 64 164 and 1103 (216, 1322);
+  // 512 x 30 x 64 186 and 1237 (161, 1209).  A long y axis gains from lines at every width.
+  const bool rod = sizeof(T) == 4 && c->ax[0].P == 0 && c->ny < 28;
+  const bool plane = (!lines || rod) && !sx.big && !sy.big &&
                      std::max(most_butterflies(c->ax[0]), most_butterflies(c->ax[1])) <= kPlaneThreads &&
                      plane_smem<T>(c) <= (size_t)max_smem() && c->tune.fft_kernels != 2;
   // which of x and y the z pass meets in a two-factor transform's order
