@@ -104,10 +104,6 @@ __device__ __forceinline__ void commit(uint64_t *bar)
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void arrive(uint64_t *bar)
-{
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // A images [mp / 128][nkb], B images [np / 64][nkb]; the CTA (x, y, z) forms rows
 // 128 x, columns 64 y over the k blocks of split z: part[z][row][col], MAG:
@@ -233,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, MAG ? 2 : 1)
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
-      if (lane == 0) arrive(&read_bar);
+      if (lane == 0) mbar_arrive(&read_bar);
     }
     if (!ok) {
       if (lane == 0) atomicExch(&fail, 1);

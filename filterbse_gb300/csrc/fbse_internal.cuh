@@ -329,7 +329,10 @@ int tc_complex_nt(fbse_ctx *c, const float2 *A, int ma, const float2 *B, int nb,
 // FP64 products on the tensor cores by exact integer slices (exactgemm.cu):
 //   out[i][j] = scale * sum_l f(A_i[l]) B_j[l] over L values of each row; rows are
 //   lda / ldb doubles apart and hold real values, or complex ones as (re, im)
-// Scratch is kept in the context; FBSE_ERR_OOM leaves nothing enqueued.
+// Every output has the accuracy of an FP64 sum, relative to sum |A_i||B_j|; its bits
+// depend on L alone.  Rows that are not finite: NaN (kExactReal, kExactConj) or the FP64
+// sum (kExactPlain).  Scratch is kept in the context (kSlotTc, which dev_alloc gives
+// back); FBSE_ERR_OOM leaves nothing enqueued.
 enum ExactKind { kExactReal, kExactPlain, kExactConj };  // real; complex; complex with f = conj
 // a product shorter than this is not worth the slicing
 constexpr long kExactMin = 2048;

@@ -1,5 +1,5 @@
 // In-register DFT helpers and the kinetic factor shared by the FFT kernels
-// (fft.cu, fft_fast.cuh) and the fused H psi kernel (hpsi_pipe.cu).
+// (fft.cu, fft_fast.cuh, fft_two.cuh) and the fused plane passes (hpsi_fused.cuh).
 #pragma once
 
 #include "fbse_internal.cuh"
