@@ -229,8 +229,8 @@ static int cgemm_nt(fbse_ctx *c, const C<T> *A, int ma, const C<T> *B, int nb, l
       return tc_complex_nt(c, A, ma, B, nb, L, scale, out);
   } else {
     // FP64: exact slices on the tensor cores; the SIMT kernel below where the
-    // product is short or their scratch does not fit
-    if (L >= kExactMin) {
+    // product is short, their scratch does not fit or an earlier wait timed out
+    if (L >= kExactMin && !c->tc_poisoned) {
       const int rc = exact_nt(c, reinterpret_cast<const double *>(A), 2 * L, ma, reinterpret_cast<const double *>(B),
                               2 * L, nb, L, kExactPlain, scale, out);
       if (rc != FBSE_ERR_OOM) return rc;

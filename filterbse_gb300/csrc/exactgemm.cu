@@ -441,8 +441,6 @@ int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, lo
              double scale, double2 *out)
 {
   using namespace ex;
-  if (c->tc_poisoned)
-    return set_err(c, FBSE_ERR_CUDA, "tensor-core path disabled: an earlier tensor-core wait timed out in this context");
   if ((double)ma * nb > 2.0e9) return set_err(c, FBSE_ERR_OOM, "exact product: too many outputs");
   const bool cplx = kind != kExactReal;
   const long K = cplx ? 2 * L : L;

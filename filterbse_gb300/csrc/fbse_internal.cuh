@@ -153,7 +153,8 @@ struct fbse_ctx {
   void *tmp = nullptr; size_t tmp_bytes = 0;     // general
   double *red = nullptr; size_t red_bytes = 0;   // reduction partials
   int *dstatus = nullptr;                        // device error flags of kernels with bounded waits
-  int tc_poisoned = 0;  // a tensor-core wait timed out: MMAs may still be in flight, the path is refused
+  int tc_poisoned = 0;  // a tensor-core wait timed out: MMAs may still be in flight, so the mixed
+                        // product is refused and FP64 ones take their SIMT kernels
   // the Rayleigh-Ritz step (ortho_diag_sigma) is running: H psi takes the mixed-radix
   // FFT kernels on every axis that the register-resident ones do not, and the
   // gather a warp per state; the autotuner's problems of these kernels say so

@@ -1129,7 +1129,7 @@ int gram_slab(fbse_ctx *c, const double *A, long na, const double *B, long nb, l
   const long stride = (long)(c->is_complex + 1) * L;
   if (na < 1 || nb < 1 || off < 0 || len < 1 || off + len > L || na > 65535 * 64L || nb > 65535 * 64L)
     return set_err(c, FBSE_ERR_ARG, "fbse_gram: sizes");
-  if (len >= kExactMin && na <= 65535 && nb <= 65535) {
+  if (len >= kExactMin && na <= 65535 && nb <= 65535 && !c->tc_poisoned) {
     const int w = c->is_complex + 1;
     // not one of the context's kept buffers: a captured graph may hold their addresses
     double2 *o = nullptr;
