@@ -333,12 +333,13 @@ int tc_complex_nt(fbse_ctx *c, const float2 *A, int ma, const float2 *B, int nb,
 // Every output has the accuracy of an FP64 sum, relative to sum |A_i||B_j|; its bits
 // depend on L alone.  Rows that are not finite: NaN (kExactReal, kExactConj) or the FP64
 // sum (kExactPlain).  Scratch is kept in the context (kSlotTc, which dev_alloc gives
-// back); FBSE_ERR_OOM leaves nothing enqueued.
+// back); FBSE_ERR_OOM leaves nothing enqueued.  out: on the device, or null for a part of
+// the scratch; out_host: receives a copy when set.
 enum ExactKind { kExactReal, kExactPlain, kExactConj };  // real; complex; complex with f = conj
 // a product shorter than this is not worth the slicing
 constexpr long kExactMin = 2048;
 int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, long ldb, int nb, long L, ExactKind kind,
-             double scale, double2 *out);
+             double scale, double2 *out, double *out_host = nullptr);
 
 // reductions / vector ops (filter.cu) ------------------------------------------
 template <typename T>

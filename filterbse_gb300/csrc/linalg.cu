@@ -1131,20 +1131,10 @@ int gram_slab(fbse_ctx *c, const double *A, long na, const double *B, long nb, l
     return set_err(c, FBSE_ERR_ARG, "fbse_gram: sizes");
   if (len >= kExactMin && na <= 65535 && nb <= 65535 && !c->tc_poisoned) {
     const int w = c->is_complex + 1;
-    // not one of the context's kept buffers: a captured graph may hold their addresses
-    double2 *o = nullptr;
-    int rx = FBSE_OK;
-    if (dev_alloc(c, &o, (size_t)na * nb * sizeof(double2)) != cudaSuccess) {
-      cudaGetLastError();
-      rx = FBSE_ERR_OOM;
-    }
-    if (!rx)
-      rx = exact_nt(c, A + off * w, stride, (int)na, B + off * w, stride, (int)nb, len,
-                    c->is_complex ? kExactConj : kExactReal, c->dv, o);
-    if (!rx && d2h(c->stream, out_host, o, (size_t)na * nb * sizeof(double2)) != cudaSuccess)
-      rx = set_err(c, FBSE_ERR_CUDA, "fbse_gram: download");
-    cudaStreamSynchronize(c->stream);
-    if (o) cudaFree(o);
+    // the result in the product's own scratch: a captured graph may hold the addresses of
+    // the context's other buffers
+    const int rx = exact_nt(c, A + off * w, stride, (int)na, B + off * w, stride, (int)nb, len,
+                            c->is_complex ? kExactConj : kExactReal, c->dv, nullptr, out_host);
     if (rx != FBSE_ERR_OOM) return rx;
   }
   const int nchunk = (int)std::min<long>(std::max<long>(1, len / 8192), 256);

@@ -20,8 +20,9 @@ def test_chunks_and_row_counts(fbse, cuda, cplx, shape, na, nb):
     a, b = (torch.tensor(rng.normal(size=(m, n * (2 if cplx else 1))), device=cuda) for m in (na, nb))
     one = ctx.gram(a, b)
     assert np.array_equal(ctx.gram(a[:2].contiguous(), b[:1].contiguous()), one[:2, :1])
-    # 64 blocks of 32 values of every row and slice are one split; 1, 2 and 5 splits a chunk
+    # a split has 32 blocks of 32 values or more, nine slices of each row: 1, 2 and 5 of the
+    # smallest splits a chunk
     rows = (na + 127) // 128 * 128 + (nb + 63) // 64 * 64 * (2 if cplx else 1)
     for splits in (1, 2, 5):
-        ctx.set_tuning(tc_image_bytes=1.2 * splits * 64 * 32 * 2 * 8 * rows)
+        ctx.set_tuning(tc_image_bytes=1.2 * splits * 32 * 32 * 2 * 9 * rows)
         assert np.array_equal(ctx.gram(a, b), one)
