@@ -2,7 +2,7 @@
 // exact integer slices:
 //   out[i][j] = scale * sum_k A[i][k] B[j][k]   (real K, or complex as real K)
 //
-// A row's values over one K split (512 to 3072 of them) share the power of two 2^e above
+// A row's values over one K split (512 to 4096 of them) share the power of two 2^e above
 // twice their largest magnitude.  x 2^-e is rounded to a 64-bit fixed-point number and cut into
 // eight signed base-256 digits d_1 .. d_8, x = 2^e sum_i d_i 2^(1 - 8 i), each a small
 // integer that BF16 holds exactly (the error-free slicing of K. Ozaki et al.,
@@ -11,16 +11,16 @@
 // stay within 2^24 and every sum is exact.  The 36 pairs with i + j <= 9 are formed.
 // Every 128 values of K the accumulators are read out and added, weighted by their
 // order, to two 64-bit integers per output, again exactly; a split ends with one
-// conversion of each to FP64 and their sum, and the splits are added in order.
+// conversion of each to FP64 and their sum; the splits are added with compensation.
 //
 // Accuracy: the pairs left out and the rounding of the digits come to less than
-// 9 x 2^-64 2^(e_a + e_b) a term, so a split is off by at most 13.5 u B, B = 2^(e_a + e_b),
+// 9 x 2^-64 2^(e_a + e_b) a term, so a split is off by at most 18 u B, B = 2^(e_a + e_b),
 // u = 2^-53 (by about 0.02 u B where the terms' errors are independent).  That is an
 // error against the rows' largest values; where these do not meet (packets apart, rows
 // of wide range) it could exceed what FP64 sums leave, which is relative to S =
 // sum |a||b|.  So S is formed as well, a ninth product of magnitudes cut to BF16, and an
 // output whose splits do not add up to 8 S >= B is summed in FP64 instead
-// (k_ex_direct): every output is within 108 u S and the roundings of adding the splits,
+// (k_ex_direct): every output is within 144 u S and a rounding or two,
 // where a running FP64 sum over K terms is within K u S.  S of a complex output is that
 // of its real and imaginary part together.  Rows with an infinity or a NaN give NaN
 // (fbse_gram) or the FP64 sum (exciton kernels).
@@ -29,11 +29,11 @@
 // 36 BF16 products at 1900 TFLOP/s are forty times that.  Measured: a complex 196 x
 // 196 product over 85184 points 115 ms on the SIMT kernel, 2.3 ms here (digits and
 // exponents 0.53, their products 1.64 or 0.98 PFLOP/s of padded tiles, 51% of the
-// measured BF16 rate, magnitudes 0.10, sums 0.05): a 128 x 64 MMA reads 192 bytes of
+// measured BF16 rate, magnitudes 0.10, sums 0.07): a 128 x 64 MMA reads 192 bytes of
 // shared memory per clock, more than there are, and the read-outs do not overlap the
 // MMAs.  fbse_gram of 128 real states of 133380 points 57 -> 0.55 ms.  Error against
-// extended precision, 2-norm, 216000 complex terms: 4e-16 (adding some 200 splits; 6e-16
-// for rows of wide range, in FP64), the SIMT kernel's 4e-16 to 3.6e-15.
+// extended precision, 2-norm, 216000 complex terms: 4e-17 to 8e-17 (6e-16 for rows of wide
+// range, in FP64), the SIMT kernel's 4e-16 to 3.6e-15.
 //
 // Operands are images of whole tiles, written once per product and moved by bulk
 // copies: 128 (A) or 64 (B) rows x 32 values x 8 slices and the magnitudes, each slice
@@ -62,14 +62,15 @@ constexpr int kBlockA = (kSlices + 1) * kTileA, kBlockB = (kSlices + 1) * kTileB
 constexpr int kDrain = 128 / kK;        // stages between read-outs
 // Stages per split, of some 2048 values: from the rows' length alone, and chunks of K are
 // whole splits added in order, so a result's bits depend neither on how many rows there
-// are nor on the room for the images.  A multiple of 76 splits of up to 96 stages: with
+// are nor on the room for the images.  A multiple of 76 splits of up to 128 stages: with
 // 1, 2, 4, .. tiles the 152 CTAs get the same number of items; 16 at least.  fbse_gram of
-// 81 x 4 and 196 x 196 complex elements of 85184 points (75 splits of 71 stages) 516 and
-// 2416 us, with 64 stages always 555 and 2600; of 2744 real points (16 stages) 164 us, with
-// 32 at least 216; of 196 x 196 complex elements of 13824 points 651, with 8 at least 717.
+// 81 x 4 and 196 x 196 complex elements of 85184 points (75 splits of 71 stages) 528 and
+// 2427 us, with 64 stages always 555 and 2600; of 1 x 1 of 133380 (76 of 110) 611, with up
+// to 96 stages 700; of 2744 real points (16 stages) 167, with 32 at least 216; of 196 x 196
+// complex elements of 13824 points 665, with 8 at least 717.
 inline long split_stages(long nkb)
 {
-  const long k = std::max(1L, (nkb + 38 * 64) / (76 * 64));
+  const long k = (nkb + 76 * 128 - 1) / (76 * 128);
   return std::max(16L, (nkb + 76 * k - 1) / (76 * k));
 }
 constexpr int kReadWarps = 8, kThreads = 32 * (2 + kReadWarps);
@@ -391,26 +392,32 @@ __global__ void __launch_bounds__(256)
 
 // out[i][j] = scale * (sum of the splits' real columns, imaginary columns), the splits
 // of all chunks in order: a chunk adds to the sums of those before it, the last one
-// scales.  bound[i][j]: 8 S - B of the splits so far; the last chunk lists the outputs
+// scales.  Compensated (W. Kahan, Comm. ACM 8 (1965) 40), so that some 100 additions leave
+// one rounding: rest[i][j] carries what o lacks.  bound[i][j]: 8 S - B of the splits so far; the last chunk lists the outputs
 // where it is negative (nan: but for those of rows that are not finite).
 __global__ void __launch_bounds__(256)
     k_ex_reduce(const double *__restrict__ part, const float *__restrict__ mag, const int *__restrict__ ea,
                 const int *__restrict__ eb, int nsplit, long mp, long np, long n1, int m, int n, bool cplx, bool first,
-                bool last, bool nan, double scale, double *__restrict__ bound, double2 *__restrict__ out,
-                int *__restrict__ list, int *__restrict__ nlist)
+                bool last, bool nan, double scale, double *__restrict__ bound, double2 *__restrict__ rest,
+                double2 *__restrict__ out, int *__restrict__ list, int *__restrict__ nlist)
 {
   const long total = (long)m * n;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
     const long i = e / n, j = e % n;
-    double2 o = first ? make_double2(0, 0) : out[e];
+    double2 o = first ? make_double2(0, 0) : out[e], r = first ? make_double2(0, 0) : rest[e];
+    auto add = [](double &sum, double &low, double p) {
+      const double y = p - low, t = sum + y;
+      low = (t - sum) - y;
+      sum = t;
+    };
     double d = first ? 0.0 : bound[e];
 #pragma unroll 12
     for (int s = 0; s < nsplit; s++) {
       const long at = ((long)s * mp + i) * np + j;
-      o.x += part[at];
+      add(o.x, r.x, part[at]);
       float g = mag[at];
       if (cplx) {
-        o.y += part[at + n1];
+        add(o.y, r.y, part[at + n1]);
         g += mag[at + n1];
       }
       const int ex = ea[s * mp + i] + eb[s * n1 + j];
@@ -422,6 +429,7 @@ __global__ void __launch_bounds__(256)
     }
     if (!last) {
       out[e] = o;
+      rest[e] = r;
       bound[e] = d;
       continue;
     }
@@ -501,12 +509,14 @@ int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, lo
   const size_t part_b = (size_t)nsplit * mp * np * sizeof(double), bound_b = ((size_t)ma * nb + 1) / 2 * sizeof(double2);
   const size_t mag_b = part_b / 2, exp_b = (size_t)nsplit * (mp + n1) * sizeof(int), list_b = (size_t)ma * nb * sizeof(int);
   const size_t out_b = out ? 0 : (size_t)ma * nb * sizeof(double2);
+  const size_t rest_b = nchunk > 1 ? (size_t)ma * nb * sizeof(double2) : 0;
   void *scratch = nullptr;
-  int rc = cached(c, kSlotTc, img_a + img_b + part_b + out_b + bound_b + mag_b + exp_b + list_b + 256, &scratch);
+  int rc = cached(c, kSlotTc, img_a + img_b + part_b + out_b + rest_b + bound_b + mag_b + exp_b + list_b + 256, &scratch);
   if (rc) return rc;
   unsigned char *ia = static_cast<unsigned char *>(scratch), *ib = ia + img_a;
   double *part = reinterpret_cast<double *>(ib + img_b);
-  double *bound = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(part) + part_b + out_b);
+  double2 *rest = reinterpret_cast<double2 *>(reinterpret_cast<unsigned char *>(part) + part_b + out_b);
+  double *bound = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(rest) + rest_b);
   if (!out) out = reinterpret_cast<double2 *>(reinterpret_cast<unsigned char *>(part) + part_b);
   float *mag = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(bound) + bound_b);
   int *ea = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(mag) + mag_b), *eb = ea + nsplit * mp;
@@ -536,8 +546,8 @@ int exact_nt(fbse_ctx *c, const double *A, long lda, int ma, const double *B, lo
                                                                                       mag, mp, np, n1, status);
     FBSE_CHECK_LAUNCH(c);
     k_ex_reduce<<<grid((long)ma * nb), 256, 0, c->stream>>>(part, mag, ea, eb, (int)ns, mp, np, n1, ma, nb, cplx, ch == 0,
-                                                             ch == nchunk - 1, kind != kExactPlain, scale, bound, out, list,
-                                                             nlist);
+                                                             ch == nchunk - 1, kind != kExactPlain, scale, bound, rest, out,
+                                                             list, nlist);
     FBSE_CHECK_LAUNCH(c);
   }
   const unsigned gd = (unsigned)std::min<long>((long)ma * nb, 152 * 8);
